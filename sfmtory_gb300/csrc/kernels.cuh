@@ -400,9 +400,20 @@ struct IntrinsicsBufs {
     int nC = 0;
     const double *poses = nullptr, *points = nullptr, *ob_xy = nullptr;
     const int *ob_img = nullptr, *ob_pt = nullptr, *cam_model = nullptr;
-    const int *cobs_start = nullptr, *cobs = nullptr;  // observations grouped by camera
-    double *cams = nullptr;                             // [nC][8] in / out
+    // Observations grouped by camera in rows of kRefineLanes (cameras with
+    // fewer than 8 have none), and the kernel's work space.
+    int rows = 0;
+    const int *row_cam = nullptr, *cam_row0 = nullptr, *row_obs = nullptr;
+    double *terms = nullptr;                 // [kRefineTerms][min(rows, kRefineChunkRows)][kRefineLanes]
+    double *lane_sum = nullptr;              // [2][kRefineTerms - 1][kRefineLanes]
+    void *state = nullptr;                   // [nC] refine_state_bytes()
+    int *active = nullptr;                   // cameras with rows
+    double *cams = nullptr;                  // [nC][8] in / out
 };
+constexpr int kRefineLanes = 128;       // lanes an observation sum is split into
+constexpr int kRefineTerms = 45;        // 44 sums and the weight
+constexpr int kRefineChunkRows = 2048;  // rows whose terms are held at once (94 MB, below the L2)
+size_t refine_state_bytes();
 void launch_refine_intrinsics(const IntrinsicsBufs &q, int max_iterations, double lambda0, int loss, double scale,
                               cudaStream_t s);
 

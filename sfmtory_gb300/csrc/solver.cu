@@ -2434,18 +2434,31 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
         cudaStream_t s = ctx.stream;
         const int nI = (int)p->num_images, nC = (int)p->num_cameras, nP = (int)p->num_points;
         const long long nO = p->num_observations;
-        // Observations grouped by camera (intrinsics.rs:125-128), in input order.
-        std::vector<int> start(nC + 1, 0), list((size_t)nO);
-        for (long long k = 0; k < nO; ++k) start[p->camera_of_image[p->obs_image[k]] + 1] += 1;
-        for (int c = 0; c < nC; ++c) start[c + 1] += start[c];
+        // Observations grouped by camera (intrinsics.rs:125-128), in input
+        // order, in rows of kRefineLanes; cameras with fewer than 8 have none.
+        std::vector<int> count(nC, 0), row0(nC + 1, 0), row_cam;
+        for (long long k = 0; k < nO; ++k) count[p->camera_of_image[p->obs_image[k]]] += 1;
+        int active = 0;
+        for (int c = 0; c < nC; ++c) {
+            const int rows = count[c] >= 8 ? div_up(count[c], kRefineLanes) : 0;
+            active += rows > 0;
+            row0[c + 1] = row0[c] + rows;
+            row_cam.insert(row_cam.end(), rows, c);
+        }
+        const int rows = row0[nC];
+        std::vector<int> row_obs((size_t)rows * kRefineLanes, -1);
         {
-            std::vector<int> fill(start.begin(), start.end() - 1);
-            for (long long k = 0; k < nO; ++k) list[fill[p->camera_of_image[p->obs_image[k]]]++] = (int)k;
+            std::vector<size_t> fill(nC);
+            for (int c = 0; c < nC; ++c) fill[c] = (size_t)row0[c] * kRefineLanes;
+            for (long long k = 0; k < nO; ++k) {
+                const int c = p->camera_of_image[p->obs_image[k]];
+                if (count[c] >= 8) row_obs[fill[c]++] = (int)k;
+            }
         }
         Arena &A = ctx.aux;
         IntrinsicsBufs q;
         double *poses = nullptr, *points = nullptr, *xy = nullptr, *cam = nullptr;
-        int *img = nullptr, *pt = nullptr, *model = nullptr, *cs = nullptr, *cl = nullptr;
+        int *img = nullptr, *pt = nullptr, *model = nullptr, *d_row_cam = nullptr, *d_row0 = nullptr, *d_row_obs = nullptr;
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 0) A.begin_sizing(); else A.commit();
             poses = A.take<double>((size_t)nI * 7);
@@ -2455,8 +2468,13 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
             img = A.take<int>(nO);
             pt = A.take<int>(nO);
             model = A.take<int>(nC);
-            cs = A.take<int>((size_t)nC + 1);
-            cl = A.take<int>(nO);
+            d_row_cam = A.take<int>(rows);
+            d_row0 = A.take<int>((size_t)nC + 1);
+            d_row_obs = A.take<int>(row_obs.size());
+            q.terms = A.take<double>((size_t)kRefineTerms * std::min(rows, kRefineChunkRows) * kRefineLanes);
+            q.lane_sum = A.take<double>((size_t)2 * (kRefineTerms - 1) * kRefineLanes);
+            q.state = A.take<char>((size_t)nC * refine_state_bytes());
+            q.active = A.take<int>(1);
         }
         put(poses, p->poses, (size_t)nI * 7, false, s);
         put(points, p->points, (size_t)nP * 3, false, s);
@@ -2465,10 +2483,13 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
         put(img, p->obs_image, nO, false, s);
         put(pt, p->obs_point, nO, false, s);
         put(model, p->camera_model, nC, false, s);
-        put_vec(cs, start, s);
-        put_vec(cl, list, s);
+        put_vec(d_row_cam, row_cam, s);
+        put_vec(d_row0, row0, s);
+        put_vec(d_row_obs, row_obs, s);
+        put(q.active, &active, 1, false, s);
         q.nC = nC; q.poses = poses; q.points = points; q.ob_xy = xy; q.ob_img = img; q.ob_pt = pt;
-        q.cam_model = model; q.cobs_start = cs; q.cobs = cl; q.cams = cam;
+        q.cam_model = model; q.rows = rows; q.row_cam = d_row_cam; q.cam_row0 = d_row0; q.row_obs = d_row_obs;
+        q.cams = cam;
         launch_refine_intrinsics(q, o->max_iterations, o->initial_lambda, o->robust_loss, o->loss_scale_px, s);
         if (nC) SFMBA_CUDA(cudaMemcpyAsync(cams, cam, sizeof(double) * 8 * (size_t)nC, cudaMemcpyDeviceToHost, s));
         SFMBA_CUDA(cudaStreamSynchronize(s));
