@@ -130,6 +130,13 @@ struct Bufs {
     long long npairs = 0;
     int ngroups = 0;
     double *S_img = nullptr;      // [nID*nID]
+    // Shared cameras of many images (launch_shared_fold_setup): the pairs of
+    // images with a common point, both directions, sorted by (camera, camera,
+    // image, image), and the slots of those cameras.
+    const uint64_t *fold_keys = nullptr;  // [fold_nkeys]
+    const int *fold_slots = nullptr;      // [fold_nslots]
+    const int *fold_shcam = nullptr;      // [nI] shared-camera index, -1: its own camera
+    int fold_nkeys = 0, fold_nslots = 0, fold_nsh = 0;
     double *S = nullptr;          // [n*n] symmetric reduced system
     double *L = nullptr;          // [n*n] Cholesky / LU factors
     double *Linv = nullptr;       // [nblocks*64*64] inverses of diagonal blocks
@@ -306,6 +313,11 @@ void launch_jacobian_probe(const JacProbe &q, bool fp32, cudaStream_t s);
 
 // ---- dense reduced system (k_dense.cu)
 void launch_schur_pairs(const Bufs &b, cudaStream_t s);
+// Slots that more images map to than this are folded through the list of image pairs (k_dense.cu).
+constexpr int kFoldList = 32;
+size_t shared_fold_temp_bytes(long long nkeys);
+void launch_shared_fold_setup(Bufs &b, uint64_t *keys, uint64_t *keys_tmp, void *temp, size_t temp_bytes,
+                              cudaStream_t s);
 void launch_fold_system(const Bufs &b, cudaStream_t s);
 void launch_fold_rhs(const Bufs &b, cudaStream_t s);  // slot-order rhs only
 void launch_cholesky(const Bufs &b, cudaStream_t s);

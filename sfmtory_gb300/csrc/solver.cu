@@ -948,6 +948,37 @@ class Solver {
         SFMBA_CUDA(cudaStreamSynchronize(s_));  // host vectors above go out of scope
     }
 
+    // Slots that many images map to and the image pairs their entries of the
+    // dense system are folded from (k_fold_shared), once per solve.
+    void setup_shared_fold() {
+        Bufs &b = b_;
+        std::vector<int> slots;
+        for (int a = 0; a < b.n; ++a)
+            if (!lay_.slot_masked[a] && lay_.slot_pre_start[a + 1] - lay_.slot_pre_start[a] > kFoldList) slots.push_back(a);
+        if (slots.empty() || b.ngroups == 0) return;
+        Arena &A = ctx_.shared;
+        uint64_t *keys = nullptr, *tmp = nullptr;
+        int *d_slots = nullptr, *d_shcam = nullptr;
+        void *temp = nullptr;
+        const size_t nk = 2 * (size_t)b.ngroups, tb = shared_fold_temp_bytes(nk);
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 0) A.begin_sizing(); else A.commit();
+            keys = A.take<uint64_t>(nk);
+            tmp = A.take<uint64_t>(nk);
+            d_slots = A.take<int>(slots.size());
+            d_shcam = A.take<int>(lay_.img_shcam.size());
+            temp = A.take<char>(tb);
+        }
+        put_vec(d_slots, slots, s_);
+        put_vec(d_shcam, lay_.img_shcam, s_);
+        b.fold_shcam = d_shcam;
+        b.fold_nsh = (int)lay_.sh_img_start.size() - 1;
+        launch_shared_fold_setup(b, keys, tmp, temp, tb, s_);
+        b.fold_slots = d_slots;
+        b.fold_nslots = (int)slots.size();
+        SFMBA_CUDA(cudaStreamSynchronize(s_));  // the host vector goes out of scope
+    }
+
     // A_c for this retry and its FP32 inverse; false (block-Jacobi alone
     // for this retry) when the sweep breaks down.
     bool factor_coarse() {
@@ -1309,6 +1340,7 @@ class Solver {
                 d_ng = P.take<int>(1);
             }
             build_pairs(b, pair_scan, ka, kb, vb, pt, ptemp, d_ng, s_);
+            if (!batch) setup_shared_fold();
             const size_t simg = batch ? (size_t)batch->simg_total : (size_t)nID * nID;
             SFMBA_CUDA(cudaMemsetAsync(b.S_img, 0, sizeof(double) * simg, s_));
         }
