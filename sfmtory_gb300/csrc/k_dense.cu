@@ -201,7 +201,7 @@ constexpr int NB = kCholNB;
 constexpr int LD = NB + 1;
 
 // Factor the diagonal block k0 (in place, lower) and write the inverse of
-// its factor to Linv (sm: two NB x LD tiles, buf: NB + 3). Sets
+// its factor to Linv (sm: two NB x LD tiles, buf: kBlkBuf). Sets
 // state->factor_failed when a pivot is not > 0 (nalgebra Cholesky::new
 // semantics: 0, negative and NaN all fail).
 __device__ __forceinline__ void chol_diag_body(double *L, int n, int k0, double *Linv, LMState *st, double *sm,
@@ -234,41 +234,17 @@ __device__ __forceinline__ void chol_diag_body(double *L, int n, int k0, double 
 
 __global__ void __launch_bounds__(256) k_chol_diag(double *L, int n, int k0, double *Linv, LMState *st) {
     extern __shared__ double sm[];
-    __shared__ double buf[NB + 3];
+    __shared__ double buf[kBlkBuf];
     chol_diag_body(L, n, k0, Linv, st, sm, buf);
 }
 
-// Panel below the diagonal block: A[r, k-block] <- A[r, k-block] Lkk^-T,
-// rows k0 + nb + blk PANEL_ROWS onwards (sm: NB + PANEL_ROWS rows of LD).
-constexpr int PANEL_ROWS = 32;
-__device__ __forceinline__ void chol_panel_body(double *L, int n, int k0, const double *Linv, const LMState *st,
-                                                int blk, double *sm) {
-    double *Li = sm;             // NB x LD
-    double *R = sm + NB * LD;    // PANEL_ROWS x LD
-    if (st->factor_failed) return;
-    const int nb = min(NB, n - k0);
-    const int r0 = k0 + nb + blk * PANEL_ROWS;
-    const int rows = min(PANEL_ROWS, n - r0);
-    if (rows <= 0) return;
-    const double *inv = Linv + (size_t)(k0 / NB) * NB * NB;
-    for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) Li[(idx / NB) * LD + idx % NB] = inv[idx];
-    for (int idx = threadIdx.x; idx < rows * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        R[r * LD + c] = L[(size_t)(r0 + r) * n + k0 + c];
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < rows * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        double s = 0.0;
-        for (int t = 0; t <= c; ++t) s += R[r * LD + t] * Li[c * LD + t];
-        L[(size_t)(r0 + r) * n + k0 + c] = s;
-    }
-}
-
+// Panel below the diagonal block k0.
 __global__ void __launch_bounds__(256) k_chol_panel(double *L, int n, int k0, const double *Linv,
                                                      const LMState *st) {
-    extern __shared__ double sm[];
-    chol_panel_body(L, n, k0, Linv, st, blockIdx.x, sm);
+    if (st->factor_failed) return;
+    const int nb = min(NB, n - k0), r0 = k0 + nb + blockIdx.x * kPanelRows;
+    if (r0 >= n) return;
+    chol_panel_rows(L, n, k0, nb, r0, min(n, r0 + kPanelRows), Linv + (size_t)(k0 / NB) * NB * NB);
 }
 
 // Tile (ti, tj), tj <= ti, of block q of a trailing update launch. part 0:
@@ -291,60 +267,18 @@ __device__ __forceinline__ void trailing_tile(long long q, int part, int &ti, in
     }
 }
 
-// Trailing update of the lower triangle: A[I,J] -= P_I P_J^T for the 64x64
-// tiles (I >= J) right of the panel. Each thread owns a 4x4 register tile.
-__device__ __forceinline__ void chol_update_body(double *L, int n, int k0, int ti, int tj, const LMState *st,
-                                                 double *sm) {
-    double *Pi = sm;            // NB x LD
-    double *Pj = sm + NB * LD;  // NB x LD
-    if (st->factor_failed) return;
-    const int nb = min(NB, n - k0);
-    const int t0 = k0 + nb;
-    const int ri = t0 + ti * NB, rj = t0 + tj * NB;
-    if (ri >= n || rj >= n) return;
-    const int mi = min(NB, n - ri), mj = min(NB, n - rj);
-    for (int idx = threadIdx.x; idx < NB * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        Pi[r * LD + c] = r < mi ? L[(size_t)(ri + r) * n + k0 + c] : 0.0;
-        Pj[r * LD + c] = r < mj ? L[(size_t)(rj + r) * n + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    for (int t = 0; t < nb; ++t) {
-        double x[4], y[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) x[a] = Pi[(ty * 4 + a) * LD + t];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) y[b] = Pj[(tx + 16 * b) * LD + t];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] += x[a] * y[b];
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int r = ty * 4 + a;
-        if (r >= mi) continue;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int c = tx + 16 * b;
-            if (c >= mj) continue;
-            if (ti == tj && c > r) continue;
-            L[(size_t)(ri + r) * n + rj + c] -= acc[a][b];
-        }
-    }
-}
-
+// Trailing update of the lower triangle right of panel k0 in TS x TS tiles:
+// block q is tile q % S^2 (S = 64 / TS) of the 64 x 64 tile q / S^2.
+template <int TS>
 __global__ void __launch_bounds__(256) k_chol_update(double *L, int n, int k0, int part, const LMState *st) {
-    extern __shared__ double sm[];
+    constexpr int S = NB / TS;
+    if (st->factor_failed) return;
     int ti, tj;
-    trailing_tile(blockIdx.x, part, ti, tj);
-    chol_update_body(L, n, k0, ti, tj, st, sm);
+    trailing_tile(blockIdx.x / (S * S), part, ti, tj);
+    const int sub = blockIdx.x % (S * S);
+    const int ri = k0 + NB + ti * NB + (sub / S) * TS, rj = k0 + NB + tj * NB + (sub % S) * TS;
+    if (ri >= n || rj > ri) return;
+    chol_update_tile<TS>(L, n, k0, ri, rj, min(TS, n - ri), min(TS, n - rj));
 }
 
 // The column loop of k_lu_pivot / k_lu_update (below) in one cooperative
@@ -705,14 +639,11 @@ void dispatch_D(int D, F &&f) {
 }
 
 const size_t kSmemTwoTiles = 2 * NB * LD * sizeof(double);
-const size_t kSmemPanel = (NB + PANEL_ROWS) * LD * sizeof(double);
 
 void set_smem_limits() {
     static bool done = false;
     if (done) return;
     SFMBA_CUDA(cudaFuncSetAttribute(k_chol_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTwoTiles));
-    SFMBA_CUDA(cudaFuncSetAttribute(k_chol_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTwoTiles));
-    SFMBA_CUDA(cudaFuncSetAttribute(k_chol_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPanel));
     SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
     done = true;
 }
@@ -866,7 +797,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
         SFMBA_LAUNCH_CHECK();
         const int rem = n - k0 - NB;
         if (rem <= 0) return;
-        k_chol_panel<<<div_up(rem, PANEL_ROWS), 256, kSmemPanel, st>>>(b.L, n, k0, b.Linv, b.state);
+        k_chol_panel<<<div_up(rem, kPanelRows), 256, 0, st>>>(b.L, n, k0, b.Linv, b.state);
         SFMBA_LAUNCH_CHECK();
         if (oz) {
             k_oz_split<<<div_up(rem, 8), 256, 0, st>>>(b.L, n, k0, slices(k0), exps(k0), b.state);
@@ -877,8 +808,10 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
         if (blocks <= 0) return;
         if (oz)
             k_oz_update<<<(unsigned)blocks, 128, kOzSmem, st>>>(b.L, n, k0, part, slices(k0), exps(k0), b.state);
+        else if (chol_tile(blocks) == 16)
+            k_chol_update<16><<<(unsigned)(16 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
         else
-            k_chol_update<<<(unsigned)blocks, 256, kSmemTwoTiles, st>>>(b.L, n, k0, part, b.state);
+            k_chol_update<32><<<(unsigned)(4 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
         SFMBA_LAUNCH_CHECK();
     };
     head(0, s);
