@@ -9,6 +9,7 @@
 // would, lib.rs:1287-1299 there).
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "camera.cuh"
@@ -459,13 +460,13 @@ __global__ void __launch_bounds__(256) k_wb_chol_solve(const double *Lall, const
 __global__ void __launch_bounds__(256) k_wb_residual(const double *Sall, const long long *s_off, const int *n_w,
                                                       const int *slot_base, const double *x, const double *rhs,
                                                       double *res, const WinState *ws) {
-    const int w = blockIdx.x;
+    const int w = blockIdx.y;
     if (!ws[w].active || ws[w].factor_failed) return;
     const int n = n_w[w];
     const double *S = Sall + s_off[w];
     const double *xw = x + slot_base[w];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < n; r += blockDim.x >> 5) {
+    const int lane = threadIdx.x & 31;
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < n; r += gridDim.x * 8) {
         double s = 0.0;
         for (int c = lane; c < n; c += 32) s += S[(size_t)r * n + c] * xw[c];
 #pragma unroll
@@ -1091,7 +1092,7 @@ void launch_wb_solve(const Bufs &b, const WinBufs &w, const double *rhs, double 
 }
 
 void launch_wb_refine(const Bufs &b, const WinBufs &w, cudaStream_t s) {
-    k_wb_residual<<<w.W, 256, 0, s>>>(b.S, w.s_off, w.n_w, w.slot_base, b.work2, w.rhs_p, b.ref_res, w.ws);
+    k_wb_residual<<<dim3(std::max(1, std::min(8, div_up(w.max_n, 8))), w.W), 256, 0, s>>>(b.S, w.s_off, w.n_w, w.slot_base, b.work2, w.rhs_p, b.ref_res, w.ws);
     SFMBA_LAUNCH_CHECK();
     launch_wb_solve(b, w, b.ref_res, b.ref_corr, s);
     if (b.n > 0) {
