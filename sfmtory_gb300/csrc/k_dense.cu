@@ -370,128 +370,132 @@ __global__ void __launch_bounds__(128, 1) k_oz_update(double *L, int n, int k0, 
                    oz_sm, fR, fC);
 }
 
-// Forward step k of L y = b: y_k = Lkk^-1 b_k, then b_r -= L[r, k-block] y_k
-// for the rows below (one warp per row).
-__global__ void __launch_bounds__(256) k_trsv_fwd(const double *L, int n, int k0, const double *Linv,
-                                                   double *b, double *y, const LMState *st) {
-    __shared__ double yk[NB];
-    __shared__ double bk[NB];
-    if (st->factor_failed) return;
-    const int nb = min(NB, n - k0);
-    const double *inv = Linv + (size_t)(k0 / NB) * NB * NB;
-    if (threadIdx.x < nb) bk[threadIdx.x] = b[k0 + threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x < nb) {  // four interleaved partial sums (FP64 latency)
-        const int r = threadIdx.x;
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int t = 0; t <= r; ++t) s[t & 3] += inv[r * NB + t] * bk[t];
-        const double v = (s[0] + s[1]) + (s[2] + s[3]);
-        yk[r] = v;
-        if (blockIdx.x == 0) y[k0 + r] = v;
+// Both triangular solves of L L^T x = rhs as a flow of 64-wide blocks over one
+// cooperative launch: block row K of the matrix belongs to thread block
+// K mod gridDim.x, which subtracts the products with y_0, y_1, .. in order as
+// they appear, multiplies by L_KK^-1 and publishes y_K; the backward sweep
+// runs the same way from the last block up the columns. A block waits only
+// for the block it needs next (a flag per block, read by one thread) instead
+// of the whole grid, and the loads of L run a block ahead of the products.
+//
+// Sums keep one fixed order: forward, entry t of a row's 64 products belongs
+// to lane t % 32 and the 32 lane sums meet in a butterfly (16, 8, 4, 2, 1),
+// of which four threads per row each take the lanes of one residue mod 4;
+// backward and with the block inverses, four interleaved sums over t % 4.
+//
+// Bound: the FP64 latency of the chain of block steps (products with the last
+// block, inverse, publication). n = 4994: 0.68 ms for both sweeps, 3.2
+// ms with a grid barrier per block step and every thread block forming the
+// products with the inverse.
+constexpr int kFlowPolls = 1 << 22;  // a few seconds; then the wait gives up
+
+// Waits (thread 0) until block k is published; false, for every thread of the
+// block, when the wait gave up (counted in LMState::wait_timeouts).
+__device__ __forceinline__ bool flow_wait(const int *ready, int k, int *ok, LMState *st) {
+    if (threadIdx.x == 0) {
+        int v = 0;
+        for (int i = 0; i < kFlowPolls && !v; ++i)
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(ready + k) : "memory");
+        if (!v) atomicAdd(&st->wait_timeouts, 1);
+        *ok = v;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rows_per_block = blockDim.x >> 5;
-    const int r = k0 + nb + blockIdx.x * rows_per_block + warp;
-    if (r >= n) return;
-    double s = 0.0;
-    for (int t = lane; t < nb; t += 32) s += L[(size_t)r * n + k0 + t] * yk[t];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) b[r] -= s;
+    return *ok != 0;
 }
 
-// Backward step k of L^T x = y: x_k = Lkk^-T y_k, then y_r -= L[k-block, r]^T x_k
-// for the rows above (one thread per row, coalesced over r).
-__global__ void __launch_bounds__(256) k_trsv_bwd(const double *L, int n, int k0, const double *Linv,
-                                                   double *y, double *x, const LMState *st) {
-    __shared__ double xk[NB];
-    __shared__ double yk[NB];
-    if (st->factor_failed) return;
-    const int nb = min(NB, n - k0);
-    const double *inv = Linv + (size_t)(k0 / NB) * NB * NB;
-    if (threadIdx.x < nb) yk[threadIdx.x] = y[k0 + threadIdx.x];
+// Publishes block k after every thread's stores to it.
+__device__ __forceinline__ void flow_publish(int *ready, int k) {
+    __threadfence();
     __syncthreads();
-    if (threadIdx.x < nb) {  // four interleaved partial sums: FP64 latency, not a 64-long chain
-        const int c = threadIdx.x;
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int r = c; r < nb; ++r) s[(r - c) & 3] += inv[r * NB + c] * yk[r];
-        const double v = (s[0] + s[1]) + (s[2] + s[3]);
-        xk[c] = v;
-        if (blockIdx.x == 0) x[k0 + c] = v;
-    }
-    __syncthreads();
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= k0) return;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int t = 0; t < nb; t += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (t + u < nb) s[u] += L[(size_t)(k0 + t + u) * n + r] * xk[t + u];
-    y[r] -= (s[0] + s[1]) + (s[2] + s[3]);
+    if (threadIdx.x == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(ready + k), "r"(1) : "memory");
 }
 
-// Both triangular solves of L L^T x = rhs in one cooperative launch: the
-// forward sweep (L y = rhs, rhs copied to `work` and updated in place) then
-// the backward sweep (L^T x = y, y updated in place), one grid barrier per
-// 64-wide block step instead of a launch. Every block forms the step's
-// diagonal product with Lkk^-1 itself from the same data (so no barrier is
-// spent on publishing it), then updates its share of the remaining rows: one
-// warp per row below in the forward sweep, one thread per row above (reading
-// L down its columns, coalesced) in the backward sweep.
-__global__ void __launch_bounds__(256) k_trsv_coop(const double *L, int n, const double *Linv, double *work,
-                                                    double *y, double *x, const LMState *st) {
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    __shared__ double vk[NB], bk[NB];
+// ready: [2 * blocks] zero; y, x: [n].
+__global__ void __launch_bounds__(256) k_trsv_flow(const double *L, int n, const double *Linv, const double *rhs,
+                                                    double *y, double *x, int *ready, LMState *st) {
+    __shared__ double Li[NB * LD], vk[NB], bk[NB], part[4][NB];
+    __shared__ int ok;
     if (st->factor_failed) return;  // read-only here: every block takes the same branch
-    const int nblk = (n + NB - 1) / NB;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + tid) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
-    for (int k = 0; k < nblk; ++k) {
-        const int k0 = k * NB, nb = min(NB, n - k0);
-        const double *inv = Linv + (size_t)k * NB * NB;
-        if (tid < nb) bk[tid] = work[k0 + tid];
-        __syncthreads();
-        if (tid < nb) {  // y_k = Lkk^-1 b_k, four interleaved partial sums
-            double s[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int t = 0; t <= tid; ++t) s[t & 3] += inv[tid * NB + t] * bk[t];
-            const double v = (s[0] + s[1]) + (s[2] + s[3]);
-            vk[tid] = v;
-            if (blockIdx.x == 0) y[k0 + tid] = v;
-        }
-        __syncthreads();
-        for (int r = k0 + nb + gw; r < n; r += nw) {
-            double s = 0.0;
-            for (int t = lane; t < nb; t += 32) s += L[(size_t)r * n + k0 + t] * vk[t];
+    const int nblk = (n + NB - 1) / NB, G = gridDim.x, tid = threadIdx.x;
+    const int q = tid >> 6, c = tid & 63;  // (sum, entry) of the interleaved sums
+    auto load_inverse = [&](int K) {
+        for (int e = tid; e < NB * NB; e += blockDim.x) Li[(e >> 6) * LD + (e & 63)] = Linv[(size_t)K * NB * NB + e];
+    };
+    for (int K = blockIdx.x; K < nblk; K += G) {
+        const int k0 = K * NB, nb = min(NB, n - k0), p = tid & 3, r = tid >> 2;
+        const double *row = L + (size_t)(k0 + min(r, nb - 1)) * n + p;
+        double acc = r < nb ? rhs[k0 + r] : 0.0, cur[16], nxt[16];
+        load_inverse(K);
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if (lane == 0) work[r] -= s;
+        for (int i = 0; i < 16; ++i) cur[i] = K > 0 ? row[4 * i] : 0.0;
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) nxt[i] = k + 1 < K ? row[(k + 1) * NB + 4 * i] : 0.0;
+            if (!flow_wait(ready, k, &ok, st)) return;
+            if (tid < NB) vk[tid] = __ldcg(y + k * NB + tid);
+            __syncthreads();
+            double d[8];  // lanes p, p + 4, .. p + 28
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                d[i] = fma(cur[i + 8], vk[4 * (i + 8) + p], fma(cur[i], vk[4 * i + p], 0.0));
+#pragma unroll
+            for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+                for (int i = 0; i < h; ++i) d[i] += d[i + h];
+            double s = d[0];
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            acc -= s;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) cur[i] = nxt[i];
+            // the next flow_wait's barrier lies between these reads of vk and its next write
         }
-        grid.sync();
+        if (p == 0) bk[r] = acc;
+        __syncthreads();
+        double s = 0.0;  // y_K = L_KK^-1 b_K
+        for (int t = q; t <= c; t += 4) s = fma(Li[c * LD + t], bk[t], s);
+        part[q][c] = s;
+        __syncthreads();
+        if (tid < nb) y[k0 + tid] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+        flow_publish(ready, K);
     }
-    for (int k = nblk - 1; k >= 0; --k) {
-        const int k0 = k * NB, nb = min(NB, n - k0);
-        const double *inv = Linv + (size_t)k * NB * NB;
-        if (tid < nb) bk[tid] = y[k0 + tid];
-        __syncthreads();
-        if (tid < nb) {  // x_k = Lkk^-T y_k
-            double s[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int r = tid; r < nb; ++r) s[(r - tid) & 3] += inv[r * NB + tid] * bk[r];
-            const double v = (s[0] + s[1]) + (s[2] + s[3]);
-            vk[tid] = v;
-            if (blockIdx.x == 0) x[k0 + tid] = v;
-        }
-        __syncthreads();
-        for (int r = blockIdx.x * blockDim.x + tid; r < k0; r += gridDim.x * blockDim.x) {
-            double s[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int t = 0; t < nb; t += 4)
+    if ((int)blockIdx.x >= nblk) return;
+    for (int K = blockIdx.x + (nblk - 1 - (int)blockIdx.x) / G * G; K >= 0; K -= G) {
+        const int k0 = K * NB, nb = min(NB, n - k0);
+        const double *col = L + k0 + min(c, nb - 1);
+        double yv = c < nb ? y[k0 + c] : 0.0, cur[16], nxt[16];
+        load_inverse(K);
+        auto fetch = [&](int k, double (&v)[16]) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (t + u < nb) s[u] += L[(size_t)(k0 + t + u) * n + r] * vk[t + u];
-            y[r] -= (s[0] + s[1]) + (s[2] + s[3]);
+            for (int i = 0; i < 16; ++i) {
+                const int t = k * NB + q + 4 * i;
+                v[i] = k > K && t < n ? col[(size_t)t * n] : 0.0;
+            }
+        };
+        fetch(nblk - 1, cur);
+        for (int k = nblk - 1; k > K; --k) {
+            fetch(k - 1, nxt);
+            if (!flow_wait(ready + nblk, k, &ok, st)) return;
+            if (tid < NB) vk[tid] = k * NB + tid < n ? __ldcg(x + k * NB + tid) : 0.0;
+            __syncthreads();
+            double s = 0.0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (k * NB + q + 4 * i < n) s = fma(cur[i], vk[q + 4 * i], s);
+            part[q][c] = s;
+            __syncthreads();
+            yv -= (part[0][c] + part[1][c]) + (part[2][c] + part[3][c]);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) cur[i] = nxt[i];
         }
-        grid.sync();
+        if (q == 0) bk[c] = yv;
+        __syncthreads();
+        double s = 0.0;  // x_K = L_KK^-T y_K
+        for (int t = c + q; t < nb; t += 4) s = fma(Li[t * LD + c], bk[t], s);
+        part[q][c] = s;
+        __syncthreads();
+        if (tid < nb) x[k0 + tid] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+        flow_publish(ready + nblk, K);
     }
 }
 
@@ -836,45 +840,18 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
 void launch_cholesky_solve(const Bufs &b, const double *rhs, double *x, cudaStream_t s) {
     const int n = b.n;
     if (n == 0) return;
-    // forward: work <- rhs (updated in place), y -> work2
-    SFMBA_CUDA(cudaMemcpyAsync(b.work, rhs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    static int cap_dev = -1, cap = 0;  // one block per SM: the diagonal products are formed per block
+    const int nblk = div_up(n, NB);
+    SFMBA_CUDA(cudaMemsetAsync(b.trsv_ready, 0, sizeof(int) * 2 * (size_t)nblk, s));
+    static int cap_dev = -1, cap = 0;  // co-resident blocks
     int dev = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     if (cap_dev != dev) {
-        int per_sm = 0, sms = 0;
-        SFMBA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_coop, 256, 0));
-        SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        cap = per_sm > 0 ? sms : 0;
+        cap = coop_capacity(k_trsv_flow, 0);
         cap_dev = dev;
     }
-    if (cap > 0) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)std::min(cap, div_up(n, 8)));
-        cfg.blockDim = dim3(256);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        SFMBA_CUDA(cudaLaunchKernelEx(&cfg, k_trsv_coop, (const double *)b.L, n, (const double *)b.Linv, b.work,
-                                      b.work2, x, (const LMState *)b.state));
-        SFMBA_LAUNCH_CHECK();
-        return;
-    }
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        const int rem = n - k0 - NB;
-        const int grid = rem > 0 ? div_up(rem, 8) : 1;
-        k_trsv_fwd<<<grid, 256, 0, s>>>(b.L, n, k0, b.Linv, b.work, b.work2, b.state);
-        SFMBA_LAUNCH_CHECK();
-    }
-    const int last = ((n - 1) / NB) * NB;
-    for (int k0 = last; k0 >= 0; k0 -= NB) {
-        const int grid = k0 > 0 ? div_up(k0, 256) : 1;
-        k_trsv_bwd<<<grid, 256, 0, s>>>(b.L, n, k0, b.Linv, b.work2, x, b.state);
-        SFMBA_LAUNCH_CHECK();
-    }
+    if (!launch_coop(k_trsv_flow, cap, nblk, 0, s, (const double *)b.L, n, (const double *)b.Linv, rhs, b.work2, x,
+                     b.trsv_ready, b.state))
+        throw Error(SFMBA_ERR_INTERNAL, "the triangular solve does not fit the GPU");
 }
 
 void launch_refine(const Bufs &b, cudaStream_t s) {

@@ -147,6 +147,7 @@ struct Bufs {
     uint16_t *oz_slices = nullptr;
     int *oz_exp = nullptr;
     int *lu_perm = nullptr;       // [n]
+    int *trsv_ready = nullptr;    // [2 * blocks of 64] published blocks of the triangular solves (single dense system)
     double *rhs = nullptr, *delta = nullptr, *diagB = nullptr, *work = nullptr, *work2 = nullptr;  // [n]
     double *ref_res = nullptr, *ref_corr = nullptr;  // [n] refinement residual and correction
     // LM bookkeeping

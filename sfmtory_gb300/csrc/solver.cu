@@ -1196,6 +1196,7 @@ class Solver {
                     b.L = A.take<double>((size_t)n * n);
                     b.Linv = A.take<double>((size_t)div_up(n, kCholNB) * kCholNB * kCholNB);
                     b.lu_perm = A.take<int>(n);
+                    b.trsv_ready = A.take<int>((size_t)2 * div_up(n, kCholNB));
                     pair_scan = A.take<long long>(nP);
                     b.oz_slices = nullptr;
                     b.oz_exp = nullptr;
@@ -1489,6 +1490,8 @@ class Solver {
                 { SFMBA_PHASE(PH_COST); launch_cost(b, true, true, s_); }
                 { SFMBA_PHASE(PH_LM); launch_accept(b, s_); launch_commit(b, s_); }
                 read_state();
+                if (solver_ == SFMBA_SOLVER_DENSE && hs.wait_timeouts)
+                    throw Error(SFMBA_ERR_INTERNAL, "a bounded wait of the triangular solve gave up");
                 if (hs.factor_failed) {
                     // LU fallback on the symmetrised system (lib.rs:1084-1092)
                     { SFMBA_PHASE(PH_LU); launch_lu_factor(b, s_); launch_lu_solve(b, s_); }
