@@ -113,6 +113,25 @@ struct LMState {
     int wait_timeouts;    // bounded waits of the TMA point pass that gave up (an internal error)
 };
 
+#ifdef __CUDACC__
+// Sums of 16 values over the 32 lanes: lane l returns the sum of v[l >> 1].
+// Each is the butterfly 16, 8, 4, 2, 1 of its value, but a level adds only the
+// half of the values that the lane keeps: 16 FP64 additions, not 80.
+__device__ __forceinline__ double warp_sum16(double (&v)[16], int lane) {
+#pragma unroll
+    for (int off = 16, m = 8; off >= 2; off >>= 1, m >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < m) {
+                const double mine = up ? v[k + m] : v[k], other = up ? v[k] : v[k + m];
+                v[k] = mine + __shfl_xor_sync(0xffffffffu, other, off);
+            }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+#endif
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace sfmba

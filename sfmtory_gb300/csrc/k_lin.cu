@@ -185,22 +185,27 @@ __global__ void __launch_bounds__(kPointInvBlock) k_point_inverse(const T *pt_C,
 }
 
 // rhs_i = -b_i + sum_o Jc~_o^T (Jx~_o h_p): the reduced right-hand side
-// (lib.rs:919-944 and :199-210). One warp per image.
-template <typename T, int D>
-__global__ void k_image_rhs(const T *rec, const int *img_start, const int *img_obs,
-                            const int *ob_pt, const T *pt_h, const unsigned char *pt_ok,
-                            const double *img_b, int nI, double *img_rhs, const unsigned char *img_live) {
+// (lib.rs:919-944 and :199-210). W warps per image (a block of 32 W threads
+// per image for W > 1, of four images for W = 1): an image's observations are
+// a chain of gathers, so few images with many observations each want several
+// warps. The FP32 form keeps one (its compensated sums have one order). 47
+// images of 2600 observations, FP64: 47 us with W = 8 against 243.
+template <typename T, int D, int W>
+__global__ void __launch_bounds__(W > 1 ? 32 * W : 128)
+    k_image_rhs(const T *rec, const int *img_start, const int *img_obs, const int *ob_pt, const T *pt_h,
+                const unsigned char *pt_ok, const double *img_b, int nI, double *img_rhs,
+                const unsigned char *img_live) {
     constexpr int RS = RecLayout<D>::kStride;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= nI) return;
-    const int i = warp;
+    __shared__ double warp_sum[W][16];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int i = W > 1 ? blockIdx.x : blockIdx.x * 4 + wl, w = W > 1 ? wl : 0;
+    if (i >= nI) return;
     if (img_live && !img_live[i]) return;
     T acc[D], comp[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) acc[c] = comp[c] = T(0);
     const int s = img_start[i], e = img_start[i + 1];
-    for (int k = s + lane; k < e; k += 32) {
+    for (int k = s + 32 * w + lane; k < e; k += 32 * W) {
         const int o = img_obs[k];
         const int p = ob_pt[o];
         if (!pt_ok[p]) continue;
@@ -211,12 +216,22 @@ __global__ void k_image_rhs(const T *rec, const int *img_start, const int *img_o
 #pragma unroll
         for (int c = 0; c < D; ++c) kahan_add(acc[c], comp[c], r[8 + c] * z0 + r[8 + D + c] * z1);
     }
+    double v[16];
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-        double v = (double)acc[c] - (double)comp[c];
+    for (int c = 0; c < 16; ++c) v[c] = c < D ? (double)acc[c] - (double)comp[c] : 0.0;
+    const double sum = warp_sum16(v, lane);  // of column lane >> 1
+    if (W == 1) {
+        if ((lane & 1) == 0 && (lane >> 1) < D)
+            img_rhs[(size_t)i * D + (lane >> 1)] = -img_b[(size_t)i * D + (lane >> 1)] + sum;
+        return;
+    }
+    if ((lane & 1) == 0) warp_sum[w][lane >> 1] = sum;
+    __syncthreads();
+    if (threadIdx.x < D) {
+        double t = 0.0;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) img_rhs[(size_t)i * D + c] = -img_b[(size_t)i * D + c] + v;
+        for (int q = 0; q < W; ++q) t += warp_sum[q][threadIdx.x];
+        img_rhs[(size_t)i * D + threadIdx.x] = -img_b[(size_t)i * D + threadIdx.x] + t;
     }
 }
 
@@ -687,19 +702,26 @@ void launch_point_inverse(const Bufs &b, cudaStream_t s) {
     SFMBA_LAUNCH_CHECK();
 }
 
+namespace {
+template <typename T, int D, int W>
+void image_rhs_w(const Bufs &b, cudaStream_t s) {
+    k_image_rhs<T, D, W><<<W > 1 ? b.nI : div_up(b.nI, 4), W > 1 ? 32 * W : 128, 0, s>>>(
+        (const T *)b.rec, b.img_start, b.img_obs, b.ob_pt, (const T *)b.pt_h, b.pt_ok, b.img_b, b.nI, b.img_rhs,
+        b.img_live);
+}
+}  // namespace
+
 void launch_image_rhs(const Bufs &b, cudaStream_t s) {
     if (b.nI == 0) return;
+    const long long per_image = b.nO / b.nI;
     dispatch_D(b.D, [&](auto dc) {
         constexpr int D = decltype(dc)::value;
-        const int warps_per_block = 4;
-        if (b.mixed)
-            k_image_rhs<float, D><<<div_up(b.nI, warps_per_block), 32 * warps_per_block, 0, s>>>(
-                (const float *)b.rec, b.img_start, b.img_obs, b.ob_pt, (const float *)b.pt_h, b.pt_ok,
-                b.img_b, b.nI, b.img_rhs, b.img_live);
-        else
-            k_image_rhs<double, D><<<div_up(b.nI, warps_per_block), 32 * warps_per_block, 0, s>>>(
-                (const double *)b.rec, b.img_start, b.img_obs, b.ob_pt, (const double *)b.pt_h,
-                b.pt_ok, b.img_b, b.nI, b.img_rhs, b.img_live);
+        // Warps by the rounds of 32 observations that a warp is left with (two
+        // at least, or the sums over the warps cost more than they save).
+        if (b.mixed) image_rhs_w<float, D, 1>(b, s);
+        else if (per_image >= 512) image_rhs_w<double, D, 8>(b, s);
+        else if (per_image >= 128) image_rhs_w<double, D, 2>(b, s);
+        else image_rhs_w<double, D, 1>(b, s);
     });
     SFMBA_LAUNCH_CHECK();
 }
