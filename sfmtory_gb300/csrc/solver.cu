@@ -1328,6 +1328,16 @@ class Solver {
             int2 *vb = nullptr;
             void *pt = nullptr;
             int *d_ng = nullptr;
+            // Chunks of the FP64 Schur reduction (also of an FP64 polish); at most
+            // one image pair per group and one chunk more than whole ones per group.
+            const bool fp64_schur = !batch && (!mixed || polish);
+            const long long max_groups = std::min<long long>(b.npairs, (long long)nI * (nI + 1) / 2);
+            if (fp64_schur) {
+                int sms = 0;
+                SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx_.device));
+                b.schur_chunk = schur_chunk_pairs(b.npairs, sms);
+                b.schur_max_chunks = (int)(b.npairs / b.schur_chunk + max_groups);
+            }
             for (int pass = 0; pass < 2; ++pass) {
                 if (pass == 0) P.begin_sizing(); else P.commit();
                 b.pairs = P.take<int2>(b.npairs);
@@ -1339,8 +1349,15 @@ class Solver {
                 vb = P.take<int2>(b.npairs + 1);
                 pt = P.take<char>(ptemp);
                 d_ng = P.take<int>(1);
+                if (fp64_schur) {
+                    b.schur_chunk_off = P.take<int>(max_groups + 1);
+                    b.schur_part_off = P.take<int>(max_groups + 1);
+                    b.schur_chunk_group = P.take<int>(b.schur_max_chunks);
+                    b.schur_part = P.take<double>((size_t)(2 * b.npairs / b.schur_chunk + 1) * D * D);
+                }
             }
             build_pairs(b, pair_scan, ka, kb, vb, pt, ptemp, d_ng, s_);
+            if (fp64_schur) launch_schur_chunks(b, pt, ptemp, s_);
             if (!batch) setup_shared_fold();
             const size_t simg = batch ? (size_t)batch->simg_total : (size_t)nID * nID;
             SFMBA_CUDA(cudaMemsetAsync(b.S_img, 0, sizeof(double) * simg, s_));
