@@ -7,16 +7,21 @@
 // (the partial Fisher-Yates shuffle restarts from the identity each time),
 // so hypothesis t depends on stream values 6t..6t+5 alone. Hypotheses are
 // therefore formed and scored in parallel, a round of B per image at a
-// time (one thread forms one 6-point DLT: conditioning test, 12 x 12
-// one-sided Jacobi SVD, polar factor, scale), one warp scores one hypothesis
-// against every correspondence, and one thread per image replays the
+// time (one thread forms one 6-point DLT: conditioning test, null vector of
+// the 12 x 12 system, polar factor, scale), one warp scores one hypothesis
+// against every correspondence, and one warp per image replays the
 // reference's adaptive loop over the round in order (best model on a strict
 // count improvement, the required iteration count re-estimated from the
 // inlier ratio) - so the chosen model and the iteration count are the
 // sequential loop's. Rounds repeat until every image's loop has ended. The
-// local refit (DLT over all inliers, a 2m x 12 Jacobi SVD with CTA-wide
-// column dot products), the never-regress checks and the two Gauss-Newton
-// polish rounds (pnp.rs:236-306) run with one CTA per image. All FP64.
+// local refit (DLT over all inliers, Householder QR of the 2m x 12 system with
+// CTA-wide column dot products), the never-regress checks and the two
+// Gauss-Newton polish rounds (pnp.rs:236-306) run with one CTA per image. All
+// FP64, but for inlier tests that FP32 with error bounds already decides.
+//
+// 512 images of 1140 correspondences, 30 % wrong: 27 -> 9 ms a call, of which
+// hypotheses 13 -> 2.1 ms (FP64 pipe: the squarings of null_vector12), scoring
+// 6 -> 0.35 ms, refit and polish 8 -> 2.9 ms, the rest copies and packing.
 #include <climits>
 #include <cstdint>
 
@@ -147,6 +152,86 @@ __device__ void jacobi_svd_serial(double *a, double *v, double *sv) {
     }
 }
 
+// Unit right singular vector v of the smallest singular value of the
+// column-major 12 x 12 matrix a, one thread (a and x, 144 entries each, are
+// scratch). Householder QR of a, the inverse X of R, and B = X X^T, whose
+// dominant eigenvector v is: B is squared (scaled to trace 1) until it has
+// rank one, sum of its squared entries = trace^2, so a ratio q of the two
+// smallest singular values converges as q^(2^k). An error in X enters v
+// divided by the ratio of the smallest to the other singular values, so v is
+// as accurate as from an SVD of a (rounding times sigma_1 / sigma_11).
+// ~6000 multiply-adds against ~80 000 of the cyclic one-sided Jacobi sweeps.
+__device__ void null_vector12(double *a, double *x, double v[12]) {
+    double scale = 0.0;
+    for (int k = 0; k < 12; ++k) {  // R in the upper triangle of a
+        double s = 0.0;
+        for (int r = k; r < 12; ++r) s = fma(a[k * 12 + r], a[k * 12 + r], s);
+        const double x0 = a[k * 12 + k];
+        if (k < 11 && s - x0 * x0 > 0.0) {
+            const double nrm = sqrt(s), alpha = x0 >= 0.0 ? -nrm : nrm, v0 = x0 - alpha;
+            const double beta = -1.0 / (alpha * v0);  // 2 / |v|^2
+            for (int j = k + 1; j < 12; ++j) {
+                double d = v0 * a[j * 12 + k];
+                for (int r = k + 1; r < 12; ++r) d = fma(a[k * 12 + r], a[j * 12 + r], d);
+                d *= beta;
+                a[j * 12 + k] = fma(-d, v0, a[j * 12 + k]);
+                for (int r = k + 1; r < 12; ++r) a[j * 12 + r] = fma(-d, a[k * 12 + r], a[j * 12 + r]);
+            }
+            a[k * 12 + k] = alpha;
+        }
+        scale = fmax(scale, fabs(a[k * 12 + k]));
+    }
+    const double tiny = scale > 0.0 ? scale * 1e-18 : 1.0;  // a zero pivot: far below rounding
+    for (int j = 0; j < 12; ++j) {  // X = R^-1, column j
+        double p = a[j * 12 + j];
+        if (fabs(p) < tiny) p = a[j * 12 + j] = tiny;
+        x[j * 12 + j] = 1.0 / p;
+        for (int i = j - 1; i >= 0; --i) {
+            double s = 0.0;
+            for (int k = i + 1; k <= j; ++k) s = fma(a[k * 12 + i], x[j * 12 + k], s);
+            x[j * 12 + i] = -s * x[i * 12 + i];
+        }
+    }
+    double tr = 0.0;
+    for (int i = 0; i < 12; ++i)
+        for (int j = 0; j <= i; ++j) {
+            double s = 0.0;
+            for (int k = i; k < 12; ++k) s = fma(x[k * 12 + i], x[k * 12 + j], s);
+            a[i * 12 + j] = a[j * 12 + i] = s;
+            if (i == j) tr += s;
+        }
+    double *B = a, *Q = x;
+    for (int it = 0;; ++it) {
+        const double inv = 1.0 / tr;
+        for (int e = 0; e < 144; ++e) B[e] *= inv;
+        if (it == 12) break;
+        double sq = 0.0;  // trace(B^2)
+        for (int i = 0; i < 12; ++i)
+            for (int j = 0; j <= i; ++j) {
+                double s = 0.0;
+#pragma unroll
+                for (int k = 0; k < 12; ++k) s = fma(B[i * 12 + k], B[j * 12 + k], s);
+                Q[i * 12 + j] = Q[j * 12 + i] = s;
+                if (i == j) sq += s;
+            }
+        double *t = B;
+        B = Q;
+        Q = t;
+        tr = sq;
+        if (!(1.0 - sq > 1e-15)) break;  // rank one (or not finite)
+    }
+    int best = 0;
+    for (int j = 1; j < 12; ++j)
+        if (B[j * 13] > B[best * 13]) best = j;
+    double nn = 0.0;
+    for (int c = 0; c < 12; ++c) {
+        v[c] = B[best * 12 + c];
+        nn = fma(v[c], v[c], nn);
+    }
+    const double s = 1.0 / sqrt(nn);
+    for (int c = 0; c < 12; ++c) v[c] *= s;
+}
+
 // The DLT rows of correspondence (X, uv) (pnp.rs:28-47) as rows r, r + 1 of
 // the column-major matrix a with leading dimension ld.
 __device__ __forceinline__ void dlt_rows(const double *X, const double *uv, double *a, int ld, int r) {
@@ -253,6 +338,67 @@ __device__ bool well_conditioned(const double *X, const long long *idx) {
     return lo / hi > 1e-3;
 }
 
+// pnp_residual(pose, X, uv) < thr, taken first in FP32 without its division,
+// |pc.xy - uv pc.z| against thr pc.z, with a bound on the rounding of every
+// term (a floating-point filter, Shewchuk 1997). What the bound leaves open
+// (some 1e-4 of the points), points next to the camera plane and anything not
+// finite go to pnp_residual itself, so the answer is its answer.
+// GB300's FP64 rate is 1/64 of FP32.
+struct InlierFilter {
+    PPose pose;
+    double thr;
+    float R[9], t[3], thr32, rmax, tmax;
+
+    __device__ InlierFilter(const PPose &p, double threshold) : pose(p), thr(threshold) {
+        // Rotation matrix of the quaternion, which pnp_residual takes as of unit
+        // length: v + 2 w (u x v) + 2 u x (u x v).
+        const PQuat &q = p.q;
+        const double xx = q.x * q.x, yy = q.y * q.y, zz = q.z * q.z;
+        const double xy = q.x * q.y, xz = q.x * q.z, yz = q.y * q.z, wx = q.w * q.x, wy = q.w * q.y, wz = q.w * q.z;
+        R[0] = (float)(1.0 - 2.0 * (yy + zz)); R[1] = (float)(2.0 * (xy - wz)); R[2] = (float)(2.0 * (xz + wy));
+        R[3] = (float)(2.0 * (xy + wz)); R[4] = (float)(1.0 - 2.0 * (xx + zz)); R[5] = (float)(2.0 * (yz - wx));
+        R[6] = (float)(2.0 * (xz - wy)); R[7] = (float)(2.0 * (yz + wx)); R[8] = (float)(1.0 - 2.0 * (xx + yy));
+        rmax = 1.f;
+        tmax = 0.f;
+        for (int k = 0; k < 9; ++k) rmax = fmaxf(rmax, fabsf(R[k]));
+        for (int k = 0; k < 3; ++k) {
+            t[k] = (float)p.t[k];
+            tmax = fmaxf(tmax, fabsf(t[k]));
+        }
+        thr32 = (float)threshold;
+    }
+
+    // a: the point and u in FP32, v likewise; X, uv: the same in FP64.
+    __device__ bool inlier(const float4 &a, float v, const double *X, const double *uv) const {
+        const float px = fmaf(R[0], a.x, fmaf(R[1], a.y, fmaf(R[2], a.z, t[0])));
+        const float py = fmaf(R[3], a.x, fmaf(R[4], a.y, fmaf(R[5], a.z, t[1])));
+        const float pz = fmaf(R[6], a.x, fmaf(R[7], a.y, fmaf(R[8], a.z, t[2])));
+        const float dx = fmaf(-a.w, pz, px), dy = fmaf(-v, pz, py);
+        const float rho = sqrtf(fmaf(dx, dx, dy * dy)), T = thr32 * pz;
+        // |pc| components are below `size` and within 6 x 2^-24 of it of their
+        // exact values (three products of rounded factors, the translation, three
+        // sums); dx, dy and T carry that error times 1 + |u|, 1 + |v| and |thr|
+        // and one more rounding each: 1e-6 of the terms covers all (2^-24 = 6e-8).
+        const float size = fmaf(rmax, fabsf(a.x) + fabsf(a.y) + fabsf(a.z), tmax);
+        const float err = 1.0e-6f * size * (2.f + fabsf(a.w) + fabsf(v) + fabsf(thr32)) + 1.0e-6f * rho;
+        if (pz > 2.0e-6f * size + 2.0e-9f) {
+            if (rho + err < T) return true;
+            if (rho - err > T) return false;
+        } else if (pz < -2.0e-6f * size && thr32 <= 3.0e38f) {
+            return false;  // behind the camera: f64::MAX is not below a finite threshold
+        }
+        return pnp_residual(pose, X, uv) < thr;
+    }
+};
+
+// FP32 copies of the correspondences for InlierFilter.
+__global__ void k_pnp_pack(const double *X, const double *uv, long long N, float4 *xyzu, float *v32) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    xyzu[i] = make_float4((float)X[3 * i], (float)X[3 * i + 1], (float)X[3 * i + 2], (float)uv[2 * i]);
+    v32[i] = (float)uv[2 * i + 1];
+}
+
 // Per-image RANSAC state (ransac.rs:90-131).
 struct PnpState {
     double best[8];      // pose of the best model (qw qx qy qz tx ty tz)
@@ -302,14 +448,9 @@ __global__ void __launch_bounds__(kPnpThreads) k_pnp_hypotheses(const long long 
     long long idx[kSample];
     for (int i = 0; i < kSample; ++i) idx[i] = get(i);
     if (!well_conditioned(Xk, idx)) return;
-    double a[12 * 12], v[12 * 12], sv[12];
+    double a[12 * 12], x[12 * 12], p[12];
     for (int i = 0; i < kSample; ++i) dlt_rows(Xk + 3 * idx[i], uvk + 2 * idx[i], a, 12, 2 * i);
-    jacobi_svd_serial<12, 12>(a, v, sv);
-    int best = 0;
-    for (int j = 1; j < 12; ++j)
-        if (sv[j] < sv[best]) best = j;
-    double p[12];
-    for (int c = 0; c < 12; ++c) p[c] = v[best * 12 + c];
+    null_vector12(a, x, p);
     PPose m;
     if (!pose_from_projection(p, m)) return;
     double *o = models + 8 * g;
@@ -325,21 +466,23 @@ __device__ __forceinline__ PPose load_pose8(const double *o) {
     return m;
 }
 
-// Inlier count of every valid hypothesis, one warp each.
+// Inlier count of every valid hypothesis, one warp each (inlier tests in FP32
+// where that decides them, see InlierFilter): 512 images x 64 hypotheses x
+// 1100 points in 0.25 ms, 6 ms with every test in FP64.
 __global__ void __launch_bounds__(256) k_pnp_score(const long long *off, const double *X, const double *uv,
-                                                   int P, int B, double thr, const double *models,
-                                                   const unsigned char *valid, long long *counts) {
+                                                   const float4 *xyzu, const float *v32, int P, int B, double thr,
+                                                   const double *models, const unsigned char *valid,
+                                                   long long *counts) {
     const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= (long long)P * B) return;
     if (!valid[w]) return;
     const int k = (int)(w / B);
     const long long s = off[k], e = off[k + 1];
-    const PPose m = load_pose8(models + 8 * w);
-    long long c = 0;
-    for (long long i = s + lane; i < e; i += 32) c += pnp_residual(m, X + 3 * i, uv + 2 * i) < thr;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    const InlierFilter f(load_pose8(models + 8 * w), thr);
+    int c = 0;
+    for (long long i = s + lane; i < e; i += 32) c += f.inlier(xyzu[i], v32[i], X + 3 * i, uv + 2 * i);
+    c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) counts[w] = c;
 }
 
@@ -347,38 +490,51 @@ __global__ void __launch_bounds__(256) k_pnp_score(const long long *off, const d
 __global__ void k_pnp_select(const long long *off, int P, int B, long long round_base, long long max_it,
                              const double *models, const unsigned char *valid, const long long *counts,
                              PnpState *st, int *active) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= P) return;
     PnpState &S = st[k];
     if (S.done) return;
     const long long n = off[k + 1] - off[k];
-    for (int h = 0; h < B; ++h) {
-        const long long limit = min(max_it, max(S.needed, 1LL));
-        if (S.iter >= limit) { S.done = 1; break; }
-        const long long t = round_base + h;
-        S.iter = t + 1;
-        const long long g = (long long)k * B + h;
-        if (!valid[g]) continue;
-        const long long c = counts[g];
-        if (!S.have || c > S.count) {
-            S.have = 1;
-            S.count = c;
-            for (int q = 0; q < 8; ++q) S.best[q] = models[8 * g + q];
-            const double ratio = fmax((double)c / (double)n, 1e-6);
-            // f64::powi(6) as binary powering: x^2 * (x^2)^2.
-            const double r2 = ratio * ratio;
-            const double denom = log(fmax(1.0 - r2 * (r2 * r2), 1e-12));
-            if (denom < 0.0) {
-                const double est = ceil(log(1.0 - 0.999) / denom);
-                if (isfinite(est) && est >= 0.0) S.needed = min((long long)est, max_it);
+    // The loop's state, the same in every lane; 32 counts are read at a time.
+    long long iter = S.iter, needed = S.needed, count = S.count, best = -1;
+    int have = S.have, done = 0;
+    for (int h0 = 0; h0 < B && !done; h0 += 32) {
+        const long long g0 = (long long)k * B + h0;
+        const long long mine = h0 + lane < B && valid[g0 + lane] ? counts[g0 + lane] : -1;  // -1: no model
+        for (int h = 0; h < min(32, B - h0); ++h) {
+            const long long limit = min(max_it, max(needed, 1LL));
+            if (iter >= limit) { done = 1; break; }
+            iter = round_base + h0 + h + 1;
+            const long long c = __shfl_sync(0xffffffffu, mine, h);
+            if (c < 0) continue;
+            if (!have || c > count) {
+                have = 1;
+                count = c;
+                best = g0 + h;
+                const double ratio = fmax((double)c / (double)n, 1e-6);
+                // f64::powi(6) as binary powering: x^2 * (x^2)^2.
+                const double r2 = ratio * ratio;
+                const double denom = log(fmax(1.0 - r2 * (r2 * r2), 1e-12));
+                if (denom < 0.0) {
+                    const double est = ceil(log(1.0 - 0.999) / denom);
+                    if (isfinite(est) && est >= 0.0) needed = min((long long)est, max_it);
+                }
             }
         }
     }
-    const long long limit = min(max_it, max(S.needed, 1LL));
-    if (!S.done && S.iter >= limit) S.done = 1;
-    if (!S.done) {
-        atomicAdd(active, 1);
-        atomicMax(active + 1, (int)min(limit - S.iter, (long long)INT_MAX));  // iterations still to run
+    const long long limit = min(max_it, max(needed, 1LL));
+    if (!done && iter >= limit) done = 1;
+    if (best >= 0 && lane < 8) S.best[lane] = models[8 * best + lane];
+    if (lane == 0) {
+        S.iter = iter;
+        S.needed = needed;
+        S.count = count;
+        S.have = have;
+        S.done = done;
+        if (!done) {
+            atomicAdd(active, 1);
+            atomicMax(active + 1, (int)min(limit - iter, (long long)INT_MAX));  // iterations still to run
+        }
     }
 }
 
@@ -387,11 +543,13 @@ template <int NV>
 __device__ void cta_sum(double (&v)[NV], double (*sh)[kPnpThreads / 32], double *out) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double x = v[q];
+    for (int q0 = 0; q0 < NV; q0 += 16) {
+        double g[16];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[q][w] = x;
+        for (int q = 0; q < 16; ++q) g[q] = q0 + q < NV ? v[min(q0 + q, NV - 1)] : 0.0;
+        const double x = warp_sum16(g, lane);
+        const int q = q0 + (lane >> 1);
+        if ((lane & 1) == 0 && q < NV) sh[q][w] = x;
     }
     __syncthreads();
     for (int q = threadIdx.x; q < NV; q += blockDim.x) {
@@ -455,8 +613,8 @@ __device__ bool lu_solve6(double a[36], const double b[6], double x[6]) {
 }
 
 struct CtaShared {
-    double red[27][kPnpThreads / 32];
-    double sums[27];
+    double red[32][kPnpThreads / 32];
+    double sums[32];
     long long cnt[kPnpThreads / 32];
     double V[144];
     double gram[3];
@@ -467,48 +625,78 @@ struct CtaShared {
 
 // pnp.rs:151-206 by one CTA: `iterations` Gauss-Newton steps over the
 // correspondences [0, n) of (X, uv) with mask[i] != 0 (mask NULL: all).
-// Upper triangle of J^T J (21) and J^T r (6) reduced per step; thread 0
-// solves and updates. sh.pose holds the pose in and out.
+// With (x, y) the normalised projection and i = 1/z the Jacobian's rows are
+//   (-xy, 1 + x^2, -y, i, 0, -x i) and (-(1 + y^2), xy, x, 0, i, -y i),
+// so the entries of J^T J and J^T r are 24 sums of few products each (~60
+// FP64 instructions a point, against ~110 for the two rows multiplied out):
+// the FP64 pipe bounds the polish. Thread 0 solves and updates. sh.pose holds
+// the pose in and out.
 __device__ void cta_refine_gn(const double *X, const double *uv, const unsigned char *mask, long long n,
                               int iterations, CtaShared &sh) {
     for (int it = 0; it < iterations; ++it) {
-        double v[27];
+        enum { XX, YY, XXQ, YYQ, XYQ, SX, SY, I1, XI, YI, XXI, YYI, XYI, XIQ, YIQ, II, XII, YII, RII, CNT,
+               G0, G1, G2, G3, G4, G5, NS };
+        double v[NS];
 #pragma unroll
-        for (int q = 0; q < 27; ++q) v[q] = 0.0;
+        for (int q = 0; q < NS; ++q) v[q] = 0.0;
         const PPose pose = sh.pose;
+        const PQuat &u = pose.q;
+        const double R[9] = {1.0 - 2.0 * (u.y * u.y + u.z * u.z), 2.0 * (u.x * u.y - u.w * u.z),
+                             2.0 * (u.x * u.z + u.w * u.y),       2.0 * (u.x * u.y + u.w * u.z),
+                             1.0 - 2.0 * (u.x * u.x + u.z * u.z), 2.0 * (u.y * u.z - u.w * u.x),
+                             2.0 * (u.x * u.z - u.w * u.y),       2.0 * (u.y * u.z + u.w * u.x),
+                             1.0 - 2.0 * (u.x * u.x + u.y * u.y)};
         for (long long i = threadIdx.x; i < n; i += blockDim.x) {
             if (mask && !mask[i]) continue;
-            double pc[3];
-            ptransform(pose, X + 3 * i, pc);
-            if (pc[2] <= 1e-9) continue;
-            const double iz = 1.0 / pc[2], x = pc[0] * iz, y = pc[1] * iz;
-            const double dr[3][3] = {{0.0, pc[2], -pc[1]}, {-pc[2], 0.0, pc[0]}, {pc[1], -pc[0], 0.0}};
-            double J[2][6];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                J[0][c] = iz * dr[0][c] - x * iz * dr[2][c];
-                J[1][c] = iz * dr[1][c] - y * iz * dr[2][c];
-            }
-            J[0][3] = iz; J[0][4] = 0.0; J[0][5] = -x * iz;
-            J[1][3] = 0.0; J[1][4] = iz; J[1][5] = -y * iz;
-            const double r0 = x - uv[2 * i], r1 = y - uv[2 * i + 1];
-            int e = 0;
-#pragma unroll
-            for (int a = 0; a < 6; ++a)
-#pragma unroll
-                for (int b = a; b < 6; ++b) v[e++] += J[0][a] * J[0][b] + J[1][a] * J[1][b];
-#pragma unroll
-            for (int a = 0; a < 6; ++a) v[21 + a] += J[0][a] * r0 + J[1][a] * r1;
+            const double X0 = X[3 * i], X1 = X[3 * i + 1], X2 = X[3 * i + 2];
+            const double pz = fma(R[6], X0, fma(R[7], X1, fma(R[8], X2, pose.t[2])));
+            if (pz <= 1e-9) continue;
+            const double px = fma(R[0], X0, fma(R[1], X1, fma(R[2], X2, pose.t[0])));
+            const double py = fma(R[3], X0, fma(R[4], X1, fma(R[5], X2, pose.t[1])));
+            const double iz = 1.0 / pz, x = px * iz, y = py * iz;
+            const double xx = x * x, yy = y * y, xy = x * y, r2 = xx + yy, q = 1.0 + r2, xi = x * iz, yi = y * iz;
+            const double r0 = x - uv[2 * i], r1 = y - uv[2 * i + 1], m = fma(x, r0, y * r1);
+            v[CNT] += 1.0;
+            v[XX] += xx;
+            v[YY] += yy;
+            v[XXQ] = fma(xx, q, v[XXQ]);
+            v[YYQ] = fma(yy, q, v[YYQ]);
+            v[XYQ] = fma(xy, 1.0 + q, v[XYQ]);
+            v[SX] += x;
+            v[SY] += y;
+            v[I1] += iz;
+            v[XI] += xi;
+            v[YI] += yi;
+            v[XXI] = fma(xx, iz, v[XXI]);
+            v[YYI] = fma(yy, iz, v[YYI]);
+            v[XYI] = fma(xy, iz, v[XYI]);
+            v[XIQ] = fma(xi, q, v[XIQ]);
+            v[YIQ] = fma(yi, q, v[YIQ]);
+            v[II] = fma(iz, iz, v[II]);
+            v[XII] = fma(xi, iz, v[XII]);
+            v[YII] = fma(yi, iz, v[YII]);
+            v[RII] = fma(xi, xi, fma(yi, yi, v[RII]));
+            v[G0] = fma(-y, m, v[G0]) - r1;
+            v[G1] = fma(x, m, v[G1]) + r0;
+            v[G2] = fma(x, r1, fma(-y, r0, v[G2]));
+            v[G3] = fma(iz, r0, v[G3]);
+            v[G4] = fma(iz, r1, v[G4]);
+            v[G5] = fma(-iz, m, v[G5]);
         }
-        cta_sum<27>(v, sh.red, sh.sums);
+        cta_sum<NS>(v, sh.red, sh.sums);
         if (threadIdx.x == 0) {
-            double A[36], rhs[6], d[6];
-            int e = 0;
-            for (int a = 0; a < 6; ++a)
-                for (int b = a; b < 6; ++b) A[a * 6 + b] = A[b * 6 + a] = sh.sums[e++];
+            const double *S = sh.sums;
+            double rhs[6], d[6];
+            double A[36] = {
+                S[CNT] + S[YY] + S[YYQ], -S[XYQ], -S[SX], -S[XYI], -(S[I1] + S[YYI]), S[YIQ],
+                -S[XYQ], S[CNT] + S[XX] + S[XXQ], -S[SY], S[I1] + S[XXI], S[XYI], -S[XIQ],
+                -S[SX], -S[SY], S[XX] + S[YY], -S[YI], S[XI], 0.0,
+                -S[XYI], S[I1] + S[XXI], -S[YI], S[II], 0.0, -S[XII],
+                -(S[I1] + S[YYI]), S[XYI], S[XI], 0.0, S[II], -S[YII],
+                S[YIQ], -S[XIQ], 0.0, -S[XII], -S[YII], S[RII]};
             for (int a = 0; a < 6; ++a) {
                 A[a * 6 + a] += 1e-9;
-                rhs[a] = -sh.sums[21 + a];
+                rhs[a] = -S[G0 + a];
             }
             bool ok = lu_solve6(A, rhs, d);
             for (int a = 0; a < 6 && ok; ++a) ok = isfinite(d[a]);
@@ -528,12 +716,12 @@ __device__ void cta_refine_gn(const double *X, const double *uv, const unsigned 
 }
 
 // Inlier count of sh.pose (and the mask, when given) by one CTA.
-__device__ long long cta_inliers(const double *X, const double *uv, long long n, double thr, unsigned char *mask,
-                                 CtaShared &sh) {
-    const PPose p = sh.pose;
+__device__ long long cta_inliers(const double *X, const double *uv, const float4 *xyzu, const float *v32, long long n,
+                                 double thr, unsigned char *mask, CtaShared &sh) {
+    const InlierFilter f(sh.pose, thr);
     long long c = 0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const bool ok = pnp_residual(p, X + 3 * i, uv + 2 * i) < thr;
+        const bool ok = f.inlier(xyzu[i], v32[i], X + 3 * i, uv + 2 * i);
         if (mask) mask[i] = ok;
         c += ok;
     }
@@ -543,19 +731,32 @@ __device__ long long cta_inliers(const double *X, const double *uv, long long n,
 // DLT over the correspondences with inl[i] != 0 (m of them, m >= 6) by one
 // CTA: the 2m x 12 system in scratch a (column-major), reduced to its 12 x 12
 // R factor by Householder reflections (column norms and the 11 column dot
-// products of each step reduced over the CTA), then thread 0 takes the
-// one-sided Jacobi SVD of R (A and R share their right singular vectors) —
-// the same steps as the oracle's restatement. Pose in sh.pose; false where
+// products of each step reduced over the CTA), then thread 0 takes
+// the null vector of R (A and R share their right singular vectors). Pose in sh.pose; false where
 // pnp_dlt returns None.
 __device__ bool cta_dlt(const double *X, const double *uv, const unsigned char *inl, long long n, long long m,
                         double *a, CtaShared &sh, long long *slot) {
     const long long M = 2 * m;
     // Rows in input order: slot[i] = rank of i among the inliers.
-    if (threadIdx.x == 0) {
-        long long r = 0;
-        for (long long i = 0; i < n; ++i) slot[i] = inl[i] ? r++ : -1;
+    {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        long long base = 0;  // inliers before this round of kPnpThreads
+        for (long long i0 = 0; i0 < n; i0 += kPnpThreads) {
+            const long long i = i0 + threadIdx.x;
+            const bool on = i < n && inl[i];
+            const unsigned b = __ballot_sync(0xffffffffu, on);
+            if (lane == 0) sh.cnt[w] = __popc(b);
+            __syncthreads();
+            long long before = base, all = 0;
+            for (int q = 0; q < kPnpThreads / 32; ++q) {
+                if (q < w) before += sh.cnt[q];
+                all += sh.cnt[q];
+            }
+            if (i < n) slot[i] = on ? before + __popc(b & ((1u << lane) - 1u)) : -1;
+            base += all;
+            __syncthreads();
+        }
     }
-    __syncthreads();
     for (long long i = threadIdx.x; i < n; i += blockDim.x)
         if (slot[i] >= 0) dlt_rows(X + 3 * i, uv + 2 * i, a, (int)M, (int)(2 * slot[i]));
     __syncthreads();
@@ -603,14 +804,9 @@ __device__ bool cta_dlt(const double *X, const double *uv, const unsigned char *
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        double R[144], V[144], sv[12];
+        double R[144], W[144], p[12];
         for (int q = 0; q < 144; ++q) R[q] = sh.V[q];
-        jacobi_svd_serial<12, 12>(R, V, sv);
-        int best = 0;
-        for (int j = 1; j < 12; ++j)
-            if (sv[j] < sv[best]) best = j;
-        double p[12];
-        for (int c = 0; c < 12; ++c) p[c] = V[best * 12 + c];
+        null_vector12(R, W, p);
         PPose out;
         sh.flag = pose_from_projection(p, out);
         if (sh.flag) sh.pose = out;
@@ -623,7 +819,8 @@ __device__ bool cta_dlt(const double *X, const double *uv, const unsigned char *
 // model, the local refit kept only if it loses no inliers, two never-regress
 // Gauss-Newton polish rounds of 10 iterations over the inliers.
 __global__ void __launch_bounds__(kPnpThreads) k_pnp_finish(const long long *off, const double *X,
-                                                            const double *uv, double thr, const PnpState *st,
+                                                            const double *uv, const float4 *xyzu,
+                                                            const float *v32, double thr, const PnpState *st,
                                                             double *dlt_scratch, long long *slot_scratch,
                                                             unsigned char *mask_a, unsigned char *mask_b,
                                                             double *poses_out, int *found_out) {
@@ -640,11 +837,11 @@ __global__ void __launch_bounds__(kPnpThreads) k_pnp_finish(const long long *off
     }
     if (threadIdx.x == 0) sh.pose = load_pose8(S.best);
     __syncthreads();
-    long long best_count = cta_inliers(Xk, uvk, n, thr, best_mask, sh);
+    long long best_count = cta_inliers(Xk, uvk, xyzu + s, v32 + s, n, thr, best_mask, sh);
     PPose best_pose = sh.pose;
     // LO refit (pnp.rs:246-268).
     if (cta_dlt(Xk, uvk, best_mask, n, best_count, dlt_scratch + 24 * s, sh, slot_scratch + s)) {
-        const long long c = cta_inliers(Xk, uvk, n, thr, trial, sh);
+        const long long c = cta_inliers(Xk, uvk, xyzu + s, v32 + s, n, thr, trial, sh);
         if (c >= best_count) {
             best_count = c;
             best_pose = sh.pose;
@@ -661,7 +858,7 @@ __global__ void __launch_bounds__(kPnpThreads) k_pnp_finish(const long long *off
         if (threadIdx.x == 0) sh.pose = best_pose;
         __syncthreads();
         cta_refine_gn(Xk, uvk, best_mask, n, 10, sh);
-        const long long c = cta_inliers(Xk, uvk, n, thr, trial, sh);
+        const long long c = cta_inliers(Xk, uvk, xyzu + s, v32 + s, n, thr, trial, sh);
         if (c < best_count) break;
         const bool converged = c == best_count;
         best_pose = sh.pose;
@@ -718,6 +915,10 @@ void launch_pnp_init(const PnpBufs &q, cudaStream_t s) {
     if (q.P == 0) return;
     k_pnp_init<<<div_up(q.P, 128), 128, 0, s>>>(q.off, q.P, q.max_it, (PnpState *)q.state);
     SFMBA_LAUNCH_CHECK();
+    if (q.N > 0) {
+        k_pnp_pack<<<div_up(q.N, 256), 256, 0, s>>>(q.X, q.uv, q.N, q.xyzu, q.v32);
+        SFMBA_LAUNCH_CHECK();
+    }
 }
 
 void launch_pnp_round(const PnpBufs &q, long long round_base, cudaStream_t s) {
@@ -725,18 +926,18 @@ void launch_pnp_round(const PnpBufs &q, long long round_base, cudaStream_t s) {
     k_pnp_hypotheses<<<div_up(total, kPnpThreads), kPnpThreads, 0, s>>>(
         q.off, q.X, q.uv, q.raw, q.P, q.B, round_base, q.max_it, (const PnpState *)q.state, q.models, q.valid);
     SFMBA_LAUNCH_CHECK();
-    k_pnp_score<<<div_up(total * 32, 256), 256, 0, s>>>(q.off, q.X, q.uv, q.P, q.B, q.thr, q.models, q.valid,
-                                                        q.counts);
+    k_pnp_score<<<div_up(total * 32, 256), 256, 0, s>>>(q.off, q.X, q.uv, q.xyzu, q.v32, q.P, q.B, q.thr, q.models,
+                                                        q.valid, q.counts);
     SFMBA_LAUNCH_CHECK();
     SFMBA_CUDA(cudaMemsetAsync(q.active, 0, 2 * sizeof(int), s));
-    k_pnp_select<<<div_up(q.P, 128), 128, 0, s>>>(q.off, q.P, q.B, round_base, q.max_it, q.models, q.valid,
+    k_pnp_select<<<div_up(q.P, 4), 128, 0, s>>>(q.off, q.P, q.B, round_base, q.max_it, q.models, q.valid,
                                                   q.counts, (PnpState *)q.state, q.active);
     SFMBA_LAUNCH_CHECK();
 }
 
 void launch_pnp_finish(const PnpBufs &q, cudaStream_t s) {
     if (q.P == 0) return;
-    k_pnp_finish<<<q.P, kPnpThreads, 0, s>>>(q.off, q.X, q.uv, q.thr, (const PnpState *)q.state, q.dlt_scratch,
+    k_pnp_finish<<<q.P, kPnpThreads, 0, s>>>(q.off, q.X, q.uv, q.xyzu, q.v32, q.thr, (const PnpState *)q.state, q.dlt_scratch,
                                              q.slot_scratch, q.mask, q.mask_trial, q.poses, q.found);
     SFMBA_LAUNCH_CHECK();
 }

@@ -450,6 +450,9 @@ struct PnpBufs {
     double thr = 0.0;
     const long long *off = nullptr;
     const double *X = nullptr, *uv = nullptr;
+    long long N = 0;
+    float4 *xyzu = nullptr;                   // [N] FP32 copies: point and u,
+    float *v32 = nullptr;                     // [N] and v
     const unsigned long long *raw = nullptr;  // [6 * max_it] xorshift64 stream
     void *state = nullptr;                    // [P] per-image RANSAC state
     double *models = nullptr;                 // [P * B][8]

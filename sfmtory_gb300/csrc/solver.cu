@@ -2225,6 +2225,8 @@ int sfmba_pnp_ransac_batched(int32_t num, const int64_t *offsets, const double *
             X = A.take<double>((size_t)N * 3 + 1);
             uv = A.take<double>((size_t)N * 2 + 1);
             raw = A.take<unsigned long long>((size_t)6 * max_iterations + 1);
+            q.xyzu = A.take<float4>((size_t)N + 1);
+            q.v32 = A.take<float>((size_t)N + 1);
             q.state = A.take<char>(pnp_state_bytes() * (size_t)num);
             q.models = A.take<double>((size_t)num * q.B * 8);
             q.valid = A.take<unsigned char>((size_t)num * q.B);
@@ -2239,6 +2241,7 @@ int sfmba_pnp_ransac_batched(int32_t num, const int64_t *offsets, const double *
             iters = A.take<long long>(num);
         }
         q.off = off;
+        q.N = N;
         q.X = X;
         q.uv = uv;
         q.raw = raw;
