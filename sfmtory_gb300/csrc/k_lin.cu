@@ -351,7 +351,8 @@ __global__ void __launch_bounds__(256) k_cost(const double *rt, const double *ca
                                               const int *cam_model, const int *ob_img,
                                               const int *ob_pt, const double2 *ob_xy, long long nO,
                                               int loss, double scale, int mode, double *partials,
-                                              long long *count_partials, float4 *rs_out) {
+                                              long long *count_partials, float4 *rs_out, const int *bad) {
+    if (bad && *bad) return;  // indices out of range: nothing is read through them
     double sum = 0.0;
     long long cnt = 0;
     for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nO;
@@ -816,7 +817,8 @@ static void cost_impl(const Bufs &b, bool trial, int mode, double *out, long lon
     auto run = [&](auto mc) {
         k_cost<decltype(mc)::value><<<kCostBlocks, 256, 0, s>>>(
             b.img_rt64, cams, points, b.cam_of_img, b.cam_model,
-            b.ob_img, b.ob_pt, b.ob_xy, b.nO, b.loss, b.loss_scale, mode, b.partials, b.count_partials, rs_out);
+            b.ob_img, b.ob_pt, b.ob_xy, b.nO, b.loss, b.loss_scale, mode, b.partials, b.count_partials, rs_out,
+            b.bad);
     };
     switch (b.uniform_model) {
     case SFMBA_SIMPLE_PINHOLE: run(std::integral_constant<int, SFMBA_SIMPLE_PINHOLE>()); break;

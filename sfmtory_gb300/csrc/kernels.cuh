@@ -160,6 +160,7 @@ struct Bufs {
     double *ref_res = nullptr, *ref_corr = nullptr;  // [n] refinement residual and correction
     // LM bookkeeping
     LMState *state = nullptr;
+    const int *bad = nullptr;     // plain cost: set by validate_problem_device, then the cost kernel reads nothing
     double *partials = nullptr;   // [kCostBlocks*2]
     double *img_rt64 = nullptr;   // [nI][12] FP64 R (row-major) and t of the poses the cost evaluates
     // Double-float copies for the FP32 path's cost (no OPENCV_FISHEYE camera):

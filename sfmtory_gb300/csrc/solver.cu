@@ -1811,25 +1811,94 @@ int sfmba_bundle_adjust_device(const sfmba_problem *p, const sfmba_options *o, s
     return st;
 }
 
+namespace {
+
+// The FP64 cost (mode 0) or the sum of residual norms (mode 1) of a host
+// problem as it is given: its arrays are uploaded and evaluated in the
+// caller's order, without the solver's sorts and layout, and the observation
+// indices are checked on the device (the kernel reads nothing through them if
+// one is out of range). False if one is: check_problem_host words the error.
+// 1.8 million observations: 0.8 ms a call, 1.75 through the solver's set-up.
+bool plain_cost(Context &ctx, const sfmba_problem *p, const sfmba_options &opt, int mode, double *sum,
+                long long *count) {
+    cudaStream_t s = ctx.stream;
+    const int nI = (int)p->num_images, nC = (int)p->num_cameras, nP = (int)p->num_points;
+    const long long nO = p->num_observations;
+    Arena &A = ctx.main;
+    Bufs b;
+    int *model = nullptr, *coi = nullptr, *bad = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 0) A.begin_sizing(); else A.commit();
+        model = A.take<int>(nC);
+        coi = A.take<int>(nI);
+        b.cams = A.take<double>((size_t)nC * 8);
+        b.poses = A.take<double>((size_t)nI * 7);
+        b.points = A.take<double>((size_t)nP * 3);
+        b.ob_img = A.take<int>(nO);
+        b.ob_pt = A.take<int>(nO);
+        b.ob_xy = A.take<double2>(nO);
+        b.state = A.take<LMState>(1);
+        b.partials = A.take<double>(kCostBlocks);
+        b.count_partials = A.take<long long>(kCostBlocks);
+        b.img_rt64 = A.take<double>((size_t)nI * 12 + 1);
+        bad = A.take<int>(1);
+    }
+    b.nI = nI; b.nC = nC; b.nP = nP; b.nO = nO;
+    b.loss = opt.robust_loss; b.loss_scale = opt.loss_scale_px;
+    b.uniform_model = nC > 0 ? p->camera_model[0] : -1;
+    for (int c = 1; c < nC; ++c)
+        if (p->camera_model[c] != b.uniform_model) { b.uniform_model = -1; break; }
+    b.cam_model = model; b.cam_of_img = coi; b.bad = bad;
+    put(b.ob_img, p->obs_image, nO, false, s);
+    put(b.ob_pt, p->obs_point, nO, false, s);
+    put(model, p->camera_model, nC, false, s);
+    put(coi, p->camera_of_image, nI, false, s);
+    SFMBA_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
+    SFMBA_CUDA(cudaMemsetAsync(b.state, 0, sizeof(LMState), s));
+    validate_problem_device(coi, model, b.ob_img, b.ob_pt, nO, nI, nC, nP, bad, s);
+    put(b.cams, p->camera_params, (size_t)nC * 8, false, s);
+    put(b.poses, p->poses, (size_t)nI * 7, false, s);
+    put(b.points, p->points, (size_t)nP * 3, false, s);
+    put(reinterpret_cast<double *>(b.ob_xy), p->obs_xy, (size_t)nO * 2, false, s);
+    if (mode == 0) launch_cost(b, false, false, s);
+    else launch_mean_error(b, s);
+    int wrong = 0;
+    SFMBA_CUDA(cudaMemcpyAsync(&wrong, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SFMBA_CUDA(cudaMemcpyAsync(ctx.h_state, b.state, sizeof(LMState), cudaMemcpyDeviceToHost, s));
+    SFMBA_CUDA(cudaStreamSynchronize(s));
+    *sum = mode == 0 ? ctx.h_state->cost : ctx.h_state->trial_cost;
+    *count = mode == 0 ? ctx.h_state->valid_obs : ctx.h_state->trial_valid_obs;
+    return wrong == 0;
+}
+
+}  // namespace
+
 static int cost_entry(const sfmba_problem *p, const sfmba_options *o, double *out, int mode) {
     return guarded([&] {
         if (!out) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "output is NULL");
         check_problem_shape(p);
-        check_problem_host(p);
         sfmba_options opt;
         sfmba_default_options(&opt);
         if (o) opt = *o;
+        if (mode == 1 || opt.precision == SFMBA_PRECISION_FP64) {
+            check_options(&opt);
+            double sum = 0.0;
+            long long count = 0;
+            if (!plain_cost(context(), p, opt, mode, &sum, &count)) {
+                check_problem_host(p);
+                throw Error(SFMBA_ERR_INVALID_ARGUMENT, "observation, image or camera index out of range");
+            }
+            *out = mode == 0 ? sum : count == 0 ? 0.0 : sum / (double)count;
+            return;
+        }
+        check_problem_host(p);
         check_options(&opt);
         Context &ctx = context();
         Solver solver(ctx, ctx.stream);
         solver.setup(p, &opt, false, false);
-        const Bufs &b = solver.bufs();
-        if (mode == 0) launch_cost(b, false, false, ctx.stream);
-        else launch_mean_error(b, ctx.stream);
+        launch_cost(solver.bufs(), false, false, ctx.stream);
         solver.read_state();
-        const LMState &hs = *ctx.h_state;
-        if (mode == 0) *out = hs.cost;
-        else *out = hs.trial_valid_obs == 0 ? 0.0 : hs.trial_cost / (double)hs.trial_valid_obs;
+        *out = ctx.h_state->cost;
     });
 }
 
