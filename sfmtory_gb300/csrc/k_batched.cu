@@ -357,24 +357,24 @@ __global__ void __launch_bounds__(256) k_wb_oz_split(const double *Lall, const l
                  (size_t)ntot * kOzK, exps + g);
 }
 
-__global__ void __launch_bounds__(128, 1) k_wb_oz_update(double *Lall, const long long *s_off, const int *n_w, int k0,
+__global__ void __launch_bounds__(128, 2) k_wb_oz_update(double *Lall, const long long *s_off, const int *n_w, int k0,
                                                          const WinState *ws, const int *row_first,
                                                          const int *slot_base, int ntot,
                                                          const __nv_bfloat16 *slices, const int *exps) {
     extern __shared__ __align__(16) unsigned char oz_sm[];
-    __shared__ double fR[kOzTile], fC[kOzTile];
+    __shared__ int xR[kOzTile], xC[kOzCols];
     const int w = blockIdx.y;
     const int n = n_w[w];
     if (!ws[w].active || ws[w].factor_failed || k0 + NB >= n) return;
-    const int t0 = k0 + NB;
-    const long long q = blockIdx.x;
+    const int t0 = k0 + NB, c0 = (blockIdx.x & 1) * kOzCols;
+    const long long q = blockIdx.x >> 1;
     int ti = (int)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
     while ((long long)(ti + 1) * (ti + 2) / 2 <= q) ++ti;
     while ((long long)ti * (ti + 1) / 2 > q) --ti;
     const int tj = (int)(q - (long long)ti * (ti + 1) / 2);
-    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile;
+    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile + c0;
     if (ri >= n || rj >= n) return;
-    const int mi = min(kOzTile, n - ri), mj = min(kOzTile, n - rj);
+    const int mi = min(kOzTile, n - ri), mj = min(kOzCols, n - rj);
     // a panel tile whose rows all start right of this column block is zero
     const int sb = slot_base[w];
     const int *rf = row_first + sb;
@@ -384,9 +384,9 @@ __global__ void __launch_bounds__(128, 1) k_wb_oz_update(double *Lall, const lon
     const int any_i = __syncthreads_or(nzi);
     const int any_j = __syncthreads_or(nzj);
     if (!any_i || !any_j) return;
-    oz_tile_update(Lall + s_off[w] + (size_t)ri * n + rj, (size_t)n, mi, mj, ti == tj,
+    oz_tile_update(Lall + s_off[w] + (size_t)ri * n + rj, (size_t)n, mi, mj, ti == tj, c0,
                    slices + (size_t)(sb + ri) * kOzK, slices + (size_t)(sb + rj) * kOzK, (size_t)ntot * kOzK,
-                   exps + sb + ri, exps + sb + rj, oz_sm, fR, fC);
+                   exps + sb + ri, exps + sb + rj, oz_sm, xR, xC);
 }
 
 // Whole triangular solve L L^T x = b of window w in one CTA (windows are at
@@ -1070,7 +1070,9 @@ void launch_wb_cholesky(const Bufs &b, const WinBufs &w, cudaStream_t s) {
             k_wb_oz_split<<<dim3(div_up(rem, 8), w.W), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.slot_base, b.n,
                                                                     (__nv_bfloat16 *)b.oz_slices, b.oz_exp);
             SFMBA_LAUNCH_CHECK();
-            k_wb_oz_update<<<grid(tiles), 128, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first, w.slot_base, b.n,
+            dim3 gu = grid(tiles);
+            gu.x *= 2;  // two halves of every 64 x 64 tile
+            k_wb_oz_update<<<gu, 128, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first, w.slot_base, b.n,
                                                     (const __nv_bfloat16 *)b.oz_slices, b.oz_exp);
         } else if (chol_tile(w.W * tiles * (tiles + 1) / 2) == 16) {
             k_wb_chol_update<16><<<grid(div_up(rem, 16)), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first,

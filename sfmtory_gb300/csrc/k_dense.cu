@@ -439,20 +439,20 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *L, int n, int k0
 // A[I, J] -= P_I P_J^T for the 64 x 64 lower tiles (I >= J) right of the
 // panel, from the slices of k_oz_split (ozaki.cuh). One 4-warp block per
 // tile; a diagonal tile writes its lower triangle.
-__global__ void __launch_bounds__(128, 1) k_oz_update(double *L, int n, int k0, int part,
+__global__ void __launch_bounds__(128, 2) k_oz_update(double *L, int n, int k0, int part,
                                                       const __nv_bfloat16 *slices, const int *exps,
                                                       const LMState *st) {
     extern __shared__ __align__(16) unsigned char oz_sm[];
-    __shared__ double fR[kOzTile], fC[kOzTile];
+    __shared__ int xR[kOzTile], xC[kOzCols];
     if (st->factor_failed) return;
-    const int t0 = k0 + NB;
+    const int t0 = k0 + NB, c0 = (blockIdx.x & 1) * kOzCols;
     int ti, tj;
-    trailing_tile(blockIdx.x, part, ti, tj);
-    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile;
+    trailing_tile(blockIdx.x >> 1, part, ti, tj);
+    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile + c0;
     if (ri >= n || rj >= n) return;
-    oz_tile_update(L + (size_t)ri * n + rj, (size_t)n, min(kOzTile, n - ri), min(kOzTile, n - rj), ti == tj,
+    oz_tile_update(L + (size_t)ri * n + rj, (size_t)n, min(kOzTile, n - ri), min(kOzCols, n - rj), ti == tj, c0,
                    slices + (size_t)ri * kOzK, slices + (size_t)rj * kOzK, (size_t)n * kOzK, exps + ri, exps + rj,
-                   oz_sm, fR, fC);
+                   oz_sm, xR, xC);
 }
 
 // Both triangular solves of L L^T x = rhs as a flow of 64-wide blocks over one
@@ -925,7 +925,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
     auto update = [&](int k0, int part, long long blocks, cudaStream_t st) {
         if (blocks <= 0) return;
         if (oz)
-            k_oz_update<<<(unsigned)blocks, 128, kOzSmem, st>>>(b.L, n, k0, part, slices(k0), exps(k0), b.state);
+            k_oz_update<<<(unsigned)(2 * blocks), 128, kOzSmem, st>>>(b.L, n, k0, part, slices(k0), exps(k0), b.state);
         else if (chol_tile(blocks) == 16)
             k_chol_update<16><<<(unsigned)(16 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
         else
