@@ -1895,10 +1895,17 @@ static int cost_entry(const sfmba_problem *p, const sfmba_options *o, double *ou
         sfmba_default_options(&opt);
         if (o) opt = *o;
         if (mode == 1 || opt.precision == SFMBA_PRECISION_FP64) {
-            check_options(&opt);
+            Context *ctx = nullptr;
+            try {
+                check_options(&opt);
+                ctx = &context();
+            } catch (...) {
+                check_problem_host(p);  // a wrong index is reported before options or a missing device
+                throw;
+            }
             double sum = 0.0;
             long long count = 0;
-            if (!plain_cost(context(), p, opt, mode, &sum, &count)) {
+            if (!plain_cost(*ctx, p, opt, mode, &sum, &count)) {
                 check_problem_host(p);
                 throw Error(SFMBA_ERR_INVALID_ARGUMENT, "observation, image or camera index out of range");
             }
