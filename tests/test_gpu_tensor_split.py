@@ -12,7 +12,7 @@ from sfmtory_gb300 import native
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("power", [-1000, -300, 0, 300, 1000])
+@pytest.mark.parametrize("power", [-960, -300, 0, 300, 960])
 @pytest.mark.parametrize("zeros", [False, True], ids=["dense", "zero-blocks"])
 def test_split_over_the_exponent_range(power, zeros):
     n = 193
