@@ -258,38 +258,16 @@ __global__ void __launch_bounds__(128) k_wb_fold(const int4 *__restrict__ fold_b
 
 // ---- batched blocked Cholesky (one matrix per window, leading dim n_w)
 
-__global__ void __launch_bounds__(256) k_wb_chol_diag(double *Lall, const long long *s_off, const int *n_w,
-                                                       double *Linv_all, const long long *linv_off, int k0,
-                                                       WinState *ws) {
-    extern __shared__ double sm[];
-    double *A = sm;
-    double *X = sm + NB * LD;
-    __shared__ double buf[kBlkBuf];
-    static_assert(LD == kBlkLD, "tile stride of chol_block_factor_invert");
-    const int w = blockIdx.x;
+// One cluster of blocks per window.
+__global__ void __cluster_dims__(kCholCluster, 1, 1) __launch_bounds__(256)
+    k_wb_chol_diag(double *Lall, const long long *s_off, const int *n_w, double *Linv_all, const long long *linv_off,
+                   int k0, WinState *ws) {
+    __shared__ CholBlock sm;
+    const int w = blockIdx.x / kCholCluster;
     const int n = n_w[w];
     if (!ws[w].active || ws[w].factor_failed || k0 >= n) return;
-    double *L = Lall + s_off[w];
-    const int nb = min(NB, n - k0);
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        A[r * LD + c] = c <= r ? L[(size_t)(k0 + r) * n + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (!chol_block_factor_invert(A, X, nb, buf)) {
-        if (tid == 0) ws[w].factor_failed = 1;
-        return;
-    }
-    for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        if (c <= r) L[(size_t)(k0 + r) * n + k0 + c] = A[r * LD + c];
-    }
-    double *out = Linv_all + linv_off[w] + (size_t)(k0 / NB) * NB * NB;
-    for (int idx = tid; idx < NB * NB; idx += blockDim.x) {
-        const int r = idx / NB, c = idx - r * NB;
-        out[idx] = (r < nb && c < nb) ? X[r * LD + c] : 0.0;
-    }
+    chol_block(Lall + s_off[w] + (size_t)k0 * n + k0, (size_t)n, min(NB, n - k0),
+               Linv_all + linv_off[w] + (size_t)(k0 / NB) * NB * NB, sm, &ws[w].factor_failed);
 }
 
 __global__ void __launch_bounds__(256) k_wb_chol_panel(double *Lall, const long long *s_off, const int *n_w,
@@ -954,12 +932,10 @@ void dispatch_D(int D, F &&f) {
     }
 }
 
-const size_t kSmemTwoTiles = 2 * NB * LD * sizeof(double);
 
 void set_smem_limits() {
     static bool done = false;
     if (done) return;
-    SFMBA_CUDA(cudaFuncSetAttribute(k_wb_chol_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTwoTiles));
     SFMBA_CUDA(cudaFuncSetAttribute(k_wb_oz_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
     done = true;
 }
@@ -1056,7 +1032,7 @@ void launch_wb_fold(const Bufs &b, const WinBufs &w, cudaStream_t s) {
 void launch_wb_cholesky(const Bufs &b, const WinBufs &w, cudaStream_t s) {
     set_smem_limits();
     for (int k0 = 0; k0 < w.max_n; k0 += NB) {
-        k_wb_chol_diag<<<w.W, 256, kSmemTwoTiles, s>>>(b.L, w.s_off, w.n_w, b.Linv, w.linv_off, k0, w.ws);
+        k_wb_chol_diag<<<kCholCluster * w.W, 256, 0, s>>>(b.L, w.s_off, w.n_w, b.Linv, w.linv_off, k0, w.ws);
         SFMBA_LAUNCH_CHECK();
         const int rem = w.max_n - k0 - NB;
         if (rem <= 0) break;

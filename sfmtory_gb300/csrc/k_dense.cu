@@ -285,42 +285,16 @@ __global__ void k_fold_rhs(const double *img_rhs, const int *pre_start, const in
 constexpr int NB = kCholNB;
 constexpr int LD = NB + 1;
 
-// Factor the diagonal block k0 (in place, lower) and write the inverse of
-// its factor to Linv (sm: two NB x LD tiles, buf: kBlkBuf). Sets
-// state->factor_failed when a pivot is not > 0 (nalgebra Cholesky::new
-// semantics: 0, negative and NaN all fail).
-__device__ __forceinline__ void chol_diag_body(double *L, int n, int k0, double *Linv, LMState *st, double *sm,
-                                               double *buf) {
-    double *A = sm;            // NB x LD
-    double *X = sm + NB * LD;  // NB x LD
-    static_assert(LD == kBlkLD, "tile stride of chol_block_factor_invert");
+// Factor the diagonal block k0 (in place, lower) and write the inverse of its
+// factor to Linv: one cluster of blocks. Sets state->factor_failed when a
+// pivot is not > 0 (nalgebra Cholesky::new semantics: 0, negative and NaN all
+// fail).
+__global__ void __cluster_dims__(kCholCluster, 1, 1) __launch_bounds__(256)
+    k_chol_diag(double *L, int n, int k0, double *Linv, LMState *st) {
+    __shared__ CholBlock sm;
     if (st->factor_failed) return;
-    const int nb = min(NB, n - k0);
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        A[r * LD + c] = c <= r ? L[(size_t)(k0 + r) * n + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (!chol_block_factor_invert(A, X, nb, buf)) {
-        if (tid == 0) st->factor_failed = 1;
-        return;
-    }
-    for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-        const int r = idx / nb, c = idx - r * nb;
-        if (c <= r) L[(size_t)(k0 + r) * n + k0 + c] = A[r * LD + c];
-    }
-    double *out = Linv + (size_t)(k0 / NB) * NB * NB;
-    for (int idx = tid; idx < NB * NB; idx += blockDim.x) {
-        const int r = idx / NB, c = idx - r * NB;
-        out[idx] = (r < nb && c < nb) ? X[r * LD + c] : 0.0;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_chol_diag(double *L, int n, int k0, double *Linv, LMState *st) {
-    extern __shared__ double sm[];
-    __shared__ double buf[kBlkBuf];
-    chol_diag_body(L, n, k0, Linv, st, sm, buf);
+    chol_block(L + (size_t)k0 * n + k0, (size_t)n, min(NB, n - k0), Linv + (size_t)(k0 / NB) * NB * NB, sm,
+               &st->factor_failed);
 }
 
 // Panel below the diagonal block k0.
@@ -727,12 +701,10 @@ void dispatch_D(int D, F &&f) {
     }
 }
 
-const size_t kSmemTwoTiles = 2 * NB * LD * sizeof(double);
 
 void set_smem_limits() {
     static bool done = false;
     if (done) return;
-    SFMBA_CUDA(cudaFuncSetAttribute(k_chol_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTwoTiles));
     SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
     done = true;
 }
@@ -911,7 +883,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
     auto exps = [&](int k0) { return b.oz_exp + ((k0 / NB) & 1) * (size_t)n; };
     // diagonal factor, panel and (tensor path) slices of block k0, on stream st
     auto head = [&](int k0, cudaStream_t st) {
-        k_chol_diag<<<1, 256, kSmemTwoTiles, st>>>(b.L, n, k0, b.Linv, b.state);
+        k_chol_diag<<<kCholCluster, 256, 0, st>>>(b.L, n, k0, b.Linv, b.state);
         SFMBA_LAUNCH_CHECK();
         const int rem = n - k0 - NB;
         if (rem <= 0) return;
