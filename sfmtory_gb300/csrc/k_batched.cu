@@ -319,52 +319,52 @@ __global__ void __launch_bounds__(256) k_wb_chol_update(double *Lall, const long
 }
 
 // Tensor-core form of the two kernels above for the mixed batch (ozaki.cuh):
-// slices and exponents of window w's panel rows (global slot index
-// slot_base[w] + row; slices [kOzSlices][ntot][64]), then the trailing tiles.
+// slices and exponents of window w's panel rows (exponents at the global slot
+// slot_base[w] + row; slices in 64-row blocks numbered as the window's diagonal
+// inverses), then the trailing tiles.
 __global__ void __launch_bounds__(256) k_wb_oz_split(const double *Lall, const long long *s_off, const int *n_w,
-                                                      int k0, const WinState *ws, const int *slot_base, int ntot,
-                                                      __nv_bfloat16 *slices, int *exps) {
+                                                      int k0, const WinState *ws, const int *slot_base,
+                                                      const long long *linv_off, __nv_bfloat16 *slices, int *exps) {
     const int w = blockIdx.y;
     const int n = n_w[w];
     if (!ws[w].active || ws[w].factor_failed || k0 >= n) return;
     const int nb = min(NB, n - k0);
     const int r = k0 + nb + blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= n) return;
-    const int g = slot_base[w] + r;
-    oz_split_row(Lall + s_off[w] + (size_t)r * n + k0, nb, threadIdx.x & 31, slices + (size_t)g * kOzK,
-                 (size_t)ntot * kOzK, exps + g);
+    oz_split_row(Lall + s_off[w] + (size_t)r * n + k0, nb, threadIdx.x & 31,
+                 slices + (linv_off[w] / (NB * NB) + r / 64) * kOzBlockElems, r & 63, exps + slot_base[w] + r);
 }
 
-__global__ void __launch_bounds__(128, 2) k_wb_oz_update(double *Lall, const long long *s_off, const int *n_w, int k0,
-                                                         const WinState *ws, const int *row_first,
-                                                         const int *slot_base, int ntot,
-                                                         const __nv_bfloat16 *slices, const int *exps) {
-    extern __shared__ __align__(16) unsigned char oz_sm[];
-    __shared__ int xR[kOzTile], xC[kOzCols];
+// Column tile q of window w's trailing matrix (of `tiles` at most) and the pair
+// of row tiles 2 p and 2 p + 1 below its diagonal tile: block (., w) counts the
+// pairs column by column.
+__global__ void __launch_bounds__(kOzThreads, 1) k_wb_oz_update(double *Lall, const long long *s_off, const int *n_w,
+                                                                int k0, WinState *ws, const int *row_first,
+                                                                const int *slot_base, const long long *linv_off,
+                                                                const __nv_bfloat16 *slices, const int *exps,
+                                                                int tiles) {
+    extern __shared__ unsigned char oz_sm[];
     const int w = blockIdx.y;
     const int n = n_w[w];
-    if (!ws[w].active || ws[w].factor_failed || k0 + NB >= n) return;
-    const int t0 = k0 + NB, c0 = (blockIdx.x & 1) * kOzCols;
-    const long long q = blockIdx.x >> 1;
-    int ti = (int)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
-    while ((long long)(ti + 1) * (ti + 2) / 2 <= q) ++ti;
-    while ((long long)ti * (ti + 1) / 2 > q) --ti;
-    const int tj = (int)(q - (long long)ti * (ti + 1) / 2);
-    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile + c0;
-    if (ri >= n || rj >= n) return;
-    const int mi = min(kOzTile, n - ri), mj = min(kOzCols, n - rj);
+    if (!ws[w].active || ws[w].factor_failed) return;
+    int p = blockIdx.x, q = 0;
+    for (; p >= (tiles - q + 1) / 2; ++q) p -= (tiles - q + 1) / 2;
+    const int rj = k0 + NB + q * kOzCols, ri = rj + p * kOzRows;
+    if (ri >= n) return;
+    const int mi = min(kOzRows, n - ri), mj = min(kOzCols, n - rj);
     // a panel tile whose rows all start right of this column block is zero
-    const int sb = slot_base[w];
+    const int sb = slot_base[w], tr = threadIdx.x;
     const int *rf = row_first + sb;
-    const int tr = threadIdx.x;
     const bool nzi = tr < mi && rf[ri + tr] <= k0 + NB - 1;
-    const bool nzj = tr >= kOzTile && tr - kOzTile < mj && rf[rj + tr - kOzTile] <= k0 + NB - 1;
+    const bool nzj = tr >= kOzRows && tr - kOzRows < mj && rf[rj + tr - kOzRows] <= k0 + NB - 1;
     const int any_i = __syncthreads_or(nzi);
     const int any_j = __syncthreads_or(nzj);
     if (!any_i || !any_j) return;
-    oz_tile_update(Lall + s_off[w] + (size_t)ri * n + rj, (size_t)n, mi, mj, ti == tj, c0,
-                   slices + (size_t)(sb + ri) * kOzK, slices + (size_t)(sb + rj) * kOzK, (size_t)ntot * kOzK,
-                   exps + sb + ri, exps + sb + rj, oz_sm, xR, xC);
+    const __nv_bfloat16 *sl = slices + linv_off[w] / (NB * NB) * kOzBlockElems;
+    const bool ok = oz_tile_update<kOzCols>(Lall + s_off[w] + (size_t)ri * n + rj, (size_t)n, mi, mj, p == 0, 0,
+                                   sl + (size_t)(ri / 64) * kOzBlockElems, sl + (size_t)(rj / 64) * kOzBlockElems,
+                                   exps + sb + ri, exps + sb + rj, oz_sm);
+    if (!ok && tr == 0) ws[w].factor_failed = 1;  // a wait gave up: the window goes to the LU
 }
 
 // Whole triangular solve L L^T x = b of window w in one CTA (windows are at
@@ -1043,13 +1043,14 @@ void launch_wb_cholesky(const Bufs &b, const WinBufs &w, cudaStream_t s) {
         const long long tiles = div_up(rem, NB);
         auto grid = [&](long long t) { return dim3((unsigned)(t * (t + 1) / 2), w.W); };
         if (b.oz_slices) {  // tensor-core update (ozaki.cuh)
-            k_wb_oz_split<<<dim3(div_up(rem, 8), w.W), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.slot_base, b.n,
-                                                                    (__nv_bfloat16 *)b.oz_slices, b.oz_exp);
+            k_wb_oz_split<<<dim3(div_up(rem, 8), w.W), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.slot_base,
+                                                                    w.linv_off, (__nv_bfloat16 *)b.oz_slices,
+                                                                    b.oz_exp);
             SFMBA_LAUNCH_CHECK();
-            dim3 gu = grid(tiles);
-            gu.x *= 2;  // two halves of every 64 x 64 tile
-            k_wb_oz_update<<<gu, 128, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first, w.slot_base, b.n,
-                                                    (const __nv_bfloat16 *)b.oz_slices, b.oz_exp);
+            const dim3 gu((unsigned)((tiles + 1) * (tiles + 1) / 4), w.W);
+            k_wb_oz_update<<<gu, kOzThreads, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first, w.slot_base,
+                                                           w.linv_off, (const __nv_bfloat16 *)b.oz_slices, b.oz_exp,
+                                                           (int)tiles);
         } else if (chol_tile(w.W * tiles * (tiles + 1) / 2) == 16) {
             k_wb_chol_update<16><<<grid(div_up(rem, 16)), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first,
                                                                        w.slot_base);

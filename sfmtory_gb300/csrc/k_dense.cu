@@ -399,34 +399,34 @@ __global__ void __launch_bounds__(256) k_lu_coop(double *A, int n, int *perm, co
 
 // ------------------------------------------------ tensor-core trailing update
 // Slices and exponents of the panel rows below the diagonal block k0 (one
-// warp per row; ozaki.cuh). slices: [kOzSlices][n][64] BF16.
+// warp per row; ozaki.cuh). slices: a block of kOzBlockElems per 64 rows.
 __global__ void __launch_bounds__(256) k_oz_split(const double *L, int n, int k0, __nv_bfloat16 *slices, int *exps,
                                                    const LMState *st) {
     if (st->factor_failed) return;
     const int nb = min(NB, n - k0);
     const int r = k0 + nb + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (r >= n) return;
-    oz_split_row(L + (size_t)r * n + k0, nb, threadIdx.x & 31, slices + (size_t)r * kOzK, (size_t)n * kOzK,
+    oz_split_row(L + (size_t)r * n + k0, nb, threadIdx.x & 31, slices + (size_t)(r / 64) * kOzBlockElems, r & 63,
                  exps + r);
 }
 
-// A[I, J] -= P_I P_J^T for the 64 x 64 lower tiles (I >= J) right of the
-// panel, from the slices of k_oz_split (ozaki.cuh). One 4-warp block per
-// tile; a diagonal tile writes its lower triangle.
-__global__ void __launch_bounds__(128, 2) k_oz_update(double *L, int n, int k0, int part,
-                                                      const __nv_bfloat16 *slices, const int *exps,
-                                                      const LMState *st) {
-    extern __shared__ __align__(16) unsigned char oz_sm[];
-    __shared__ int xR[kOzTile], xC[kOzCols];
+// A[I, J] -= P_I P_J^T right of the panel, from the slices of k_oz_split
+// (ozaki.cuh): block (p, q) has columns tj0 * 64 + q * NC .. of the trailing
+// matrix and the pair of 64-row tiles 2 p and 2 p + 1 below their diagonal
+// tile.
+template <int NC>
+__global__ void __launch_bounds__(kOzThreads, 1) k_oz_update(double *L, int n, int k0, int tj0,
+                                                             const __nv_bfloat16 *slices, const int *exps,
+                                                             LMState *st) {
+    extern __shared__ unsigned char oz_sm[];
     if (st->factor_failed) return;
-    const int t0 = k0 + NB, c0 = (blockIdx.x & 1) * kOzCols;
-    int ti, tj;
-    trailing_tile(blockIdx.x >> 1, part, ti, tj);
-    const int ri = t0 + ti * kOzTile, rj = t0 + tj * kOzTile + c0;
+    const int c0 = (int)blockIdx.y * NC % 64;
+    const int rj = k0 + NB + tj0 * 64 + (int)blockIdx.y * NC, ri = rj - c0 + (int)blockIdx.x * kOzRows;
     if (ri >= n || rj >= n) return;
-    oz_tile_update(L + (size_t)ri * n + rj, (size_t)n, min(kOzTile, n - ri), min(kOzCols, n - rj), ti == tj, c0,
-                   slices + (size_t)ri * kOzK, slices + (size_t)rj * kOzK, (size_t)n * kOzK, exps + ri, exps + rj,
-                   oz_sm, xR, xC);
+    const bool ok = oz_tile_update<NC>(L + (size_t)ri * n + rj, (size_t)n, min(kOzRows, n - ri), min(NC, n - rj),
+                                       blockIdx.x == 0, c0, slices + (size_t)(ri / 64) * kOzBlockElems,
+                                       slices + (size_t)(rj / 64) * kOzBlockElems, exps + ri, exps + rj, oz_sm);
+    if (!ok && threadIdx.x == 0) st->factor_failed = 1;  // a wait gave up: the system goes to the LU
 }
 
 // Both triangular solves of L L^T x = rhs as a flow of 64-wide blocks over one
@@ -705,7 +705,8 @@ void dispatch_D(int D, F &&f) {
 void set_smem_limits() {
     static bool done = false;
     if (done) return;
-    SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
+    SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
+    SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
     done = true;
 }
 
@@ -878,7 +879,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
     const int n = b.n;
     if (n == 0) return;
     const bool oz = b.oz_slices != nullptr;
-    const size_t slice_elems = (size_t)kOzSlices * n * kOzK;
+    const size_t slice_elems = div_up(n, 64) * kOzBlockElems;
     auto slices = [&](int k0) { return (__nv_bfloat16 *)b.oz_slices + ((k0 / NB) & 1) * slice_elems; };
     auto exps = [&](int k0) { return b.oz_exp + ((k0 / NB) & 1) * (size_t)n; };
     // diagonal factor, panel and (tensor path) slices of block k0, on stream st
@@ -894,11 +895,19 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
             SFMBA_LAUNCH_CHECK();
         }
     };
-    auto update = [&](int k0, int part, long long blocks, cudaStream_t st) {
-        if (blocks <= 0) return;
-        if (oz)
-            k_oz_update<<<(unsigned)(2 * blocks), 128, kOzSmem, st>>>(b.L, n, k0, part, slices(k0), exps(k0), b.state);
-        else if (chol_tile(blocks) == 16)
+    auto update = [&](int k0, int part, cudaStream_t st) {
+        const int tiles = div_up(n - k0 - NB, NB);
+        const long long blocks = part == 1 ? tiles : (tiles - 1LL) * tiles / 2;
+        if (oz) {
+            // The next block's column is on the chain and few tiles: narrow ones (15 us
+            // for n = 2560 against 22).
+            if (part == 1)
+                k_oz_update<32><<<dim3(div_up(tiles, 2), 2), kOzThreads, kOzSmem, st>>>(b.L, n, k0, 0, slices(k0),
+                                                                                       exps(k0), b.state);
+            else
+                k_oz_update<64><<<dim3(tiles / 2, tiles - 1), kOzThreads, kOzSmem, st>>>(b.L, n, k0, 1, slices(k0),
+                                                                                        exps(k0), b.state);
+        } else if (chol_tile(blocks) == 16)
             k_chol_update<16><<<(unsigned)(16 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
         else
             k_chol_update<32><<<(unsigned)(4 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
@@ -908,7 +917,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
     for (int k0 = 0; k0 + NB < n; k0 += NB) {
         const long long tiles = div_up(n - k0 - NB, NB);
         const int k1 = k0 + NB;
-        update(k0, 1, tiles, s);  // tile column of block k1
+        update(k0, 1, s);  // tile column of block k1
         if (tiles == 1) {
             head(k1, s);
             continue;
@@ -918,7 +927,7 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
         SFMBA_CUDA(cudaStreamWaitEvent(la.s2, la.col_done, 0));
         head(k1, la.s2);
         SFMBA_CUDA(cudaEventRecord(la.next_ready, la.s2));
-        update(k0, 2, (tiles - 1) * tiles / 2, s);
+        update(k0, 2, s);
         SFMBA_CUDA(cudaStreamWaitEvent(s, la.next_ready, 0));
     }
 }

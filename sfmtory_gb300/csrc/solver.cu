@@ -1201,7 +1201,7 @@ class Solver {
                     b.oz_slices = nullptr;
                     b.oz_exp = nullptr;
                     if (mixed && !o->dense_fp64_fma) {  // tensor-core trailing updates (ozaki.cuh)
-                        b.oz_slices = A.take<uint16_t>((size_t)kOzSlices * n * kOzK);
+                        b.oz_slices = A.take<uint16_t>((size_t)(batch->linv_total / (kCholNB * kCholNB)) * kOzBlockElems);
                         b.oz_exp = A.take<int>(n);
                     }
                 } else if (solver_ == SFMBA_SOLVER_DENSE) {
@@ -1215,7 +1215,7 @@ class Solver {
                     b.oz_slices = nullptr;
                     b.oz_exp = nullptr;
                     if (mixed && !o->dense_fp64_fma) {  // tensor-core trailing updates (ozaki.cuh)
-                        b.oz_slices = A.take<uint16_t>((size_t)2 * kOzSlices * n * kOzK);
+                        b.oz_slices = A.take<uint16_t>((size_t)2 * div_up(n, 64) * kOzBlockElems);
                         b.oz_exp = A.take<int>((size_t)2 * n);
                     }
                 } else {
@@ -2789,7 +2789,7 @@ int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_u
         b.Linv = (double *)dev_alloc((size_t)div_up((int)n, kCholNB) * kCholNB * kCholNB * sizeof(double));
         b.state = (LMState *)dev_alloc(sizeof(LMState));
         if (tensor_update) {
-            b.oz_slices = (uint16_t *)dev_alloc((size_t)2 * kOzSlices * n * kOzK * sizeof(uint16_t));
+            b.oz_slices = (uint16_t *)dev_alloc((size_t)2 * div_up((int)n, 64) * kOzBlockElems * sizeof(uint16_t));
             b.oz_exp = (int *)dev_alloc((size_t)2 * n * sizeof(int));
         }
         int failed = 0;
