@@ -796,77 +796,151 @@ __global__ void k_wb_lu_update(double *Lall, const long long *s_off, const int *
     A[(size_t)r * n + c] -= A[(size_t)r * n + k] * A[(size_t)k * n + c];
 }
 
-// The column loop of the two kernels above in one cooperative launch: per
-// column k, the failed windows' pivots (a block per window, grid-stride),
-// a grid barrier, the rank-1 updates of all their trailing rows (a block per
-// (window, row), grid-stride), a grid barrier: 2 barriers per column
-// instead of 2 launches. Same arithmetic in the same order.
+// The column loop of the two kernels above in one cooperative launch with one
+// grid barrier per column. The rows of all failed windows are numbered one
+// window after another and dealt to the blocks in runs. No row is swapped:
+// every block keeps the order of the rows of its windows (order[p]: the row at
+// place p), finds the pivot of column k among the places from k on by itself
+// (the first maximum, as above) and updates its own rows that are not pivots
+// yet, a row a warp. A row's multiplier is stored after the next barrier: other
+// blocks may still be searching the column it replaces. Same operations on
+// every entry in the same order, so the same factors; perm receives the order.
+//
+// Bound: the chain of a column (barrier, column, pivot, division, row), not
+// bandwidth: 7.8 ms for one 890-unknown window with its solve, against 13.1 with
+// pivots, swaps and divisions by one block between two barriers.
+struct LuRow {
+    double l;   // multiplier to store ..
+    int lcol;   // .. in this column, -1: none
+    int active; // not a pivot yet
+};
+struct LuWindow {
+    int w, n, order, first, lo, hi;  // its order's place in shared memory; its owned rows lo..hi, first: of the block's
+};
+
+size_t lu_coop_smem(long long rows, int max_n) {
+    return (size_t)rows * (sizeof(LuRow) + sizeof(int)) + (size_t)(rows + 2) * sizeof(LuWindow) +
+           (size_t)2 * max_n * sizeof(int);
+}
+
 __global__ void __launch_bounds__(256) k_wb_lu_coop(double *Lall, const long long *s_off, const int *n_w,
                                                      const int *slot_base, int *perm_all, const int *list, int nf,
-                                                     int max_n) {
+                                                     int max_n, int max_rows) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    __shared__ double bv[256];
-    __shared__ int bi[256];
-    const int tid = threadIdx.x;
-    for (int k = 0; k < max_n; ++k) {
-        for (int f = blockIdx.x; f < nf; f += gridDim.x) {
-            const int w = list[f];
-            const int n = n_w[w];
-            if (k >= n) continue;
-            double *A = Lall + s_off[w];
-            int *perm = perm_all + slot_base[w];
-            double best = -1.0;
-            int besti = k;
-            for (int r = k + tid; r < n; r += blockDim.x) {
-                const double v = fabs(A[(size_t)r * n + k]);
-                if (v > best) { best = v; besti = r; }
+    extern __shared__ __align__(16) unsigned char lu_sm[];
+    LuRow *rows = reinterpret_cast<LuRow *>(lu_sm);
+    LuWindow *wins = reinterpret_cast<LuWindow *>(rows + max_rows);
+    int *orders = reinterpret_cast<int *>(wins + max_rows + 2);
+    __shared__ unsigned long long best_key[8];
+    __shared__ int best_at[8], nwin;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        long long total = 0;
+        for (int f = 0; f < nf; ++f) total += n_w[list[f]];
+        const long long per = (total + gridDim.x - 1) / gridDim.x;
+        const long long lo = min(total, per * blockIdx.x), hi = min(total, lo + per);
+        int c = 0, at = 0;
+        long long base = 0;
+        for (int f = 0; f < nf && base < hi; ++f) {
+            const int w = list[f], n = n_w[w];
+            if (n > 0 && base + n > lo) {
+                const int a = (int)(max(lo, base) - base), e = (int)(min(hi, base + n) - base);
+                wins[c++] = {w, n, at, (int)(max(lo, base) - lo), a, e};
+                at += n;
             }
-            bv[tid] = best;
-            bi[tid] = besti;
-            __syncthreads();
-            for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-                if (tid < h) {
-                    const double o = bv[tid + h];
-                    const int oi = bi[tid + h];
-                    if (o > bv[tid] || (o == bv[tid] && oi < bi[tid])) { bv[tid] = o; bi[tid] = oi; }
-                }
-                __syncthreads();
-            }
-            const int piv = bi[0];
-            const double diag = A[(size_t)piv * n + k];
-            if (diag != 0.0) {
-                if (piv != k)
-                    for (int c = tid; c < n; c += blockDim.x) {
-                        const double t = A[(size_t)k * n + c];
-                        A[(size_t)k * n + c] = A[(size_t)piv * n + c];
-                        A[(size_t)piv * n + c] = t;
-                    }
-                __syncthreads();
-                for (int r = k + 1 + tid; r < n; r += blockDim.x) A[(size_t)r * n + k] /= diag;
-            }
-            if (tid == 0) perm[k] = diag != 0.0 ? piv : -1;
-            __syncthreads();  // bv / bi are reused by the next window
+            base += n;
         }
-        grid.sync();
-        const int m = max_n - k - 1;
-        if (m <= 0) break;
-        for (long long q = blockIdx.x; q < (long long)nf * m; q += gridDim.x) {
-            const int f = (int)(q / m), r = k + 1 + (int)(q - (long long)f * m);
-            const int w = list[f];
-            const int n = n_w[w];
-            if (r >= n || perm_all[slot_base[w] + k] < 0) continue;
-            double *A = Lall + s_off[w];
-            const double lrk = A[(size_t)r * n + k];
-            for (int c = k + 1 + tid; c < n; c += blockDim.x) A[(size_t)r * n + c] -= lrk * A[(size_t)k * n + c];
+        nwin = c;
+    }
+    __syncthreads();
+    for (int i = 0; i < nwin; ++i) {
+        const LuWindow W = wins[i];
+        for (int p = tid; p < W.n; p += blockDim.x) orders[W.order + p] = p;
+        for (int r = W.lo + tid; r < W.hi; r += blockDim.x) rows[W.first + r - W.lo] = {0.0, -1, 1};
+    }
+    __syncthreads();
+    for (int k = 0; k <= max_n; ++k) {  // the last turn stores the last multipliers
+        for (int i = 0; i < nwin; ++i) {
+            const LuWindow W = wins[i];
+            if (k > W.n) continue;
+            double *A = Lall + s_off[W.w];
+            LuRow *mine = rows + W.first - W.lo;
+            int *order = orders + W.order;
+            for (int r = W.lo + tid; r < W.hi; r += blockDim.x)
+                if (mine[r].lcol >= 0) {
+                    A[(size_t)r * W.n + mine[r].lcol] = mine[r].l;
+                    mine[r].lcol = -1;
+                }
+            if (k == W.n) continue;
+            // The first maximum: |a| as an integer, 0 for NaN, which no comparison prefers.
+            unsigned long long key = 0;
+            int at = k;
+            for (int p = k + tid; p < W.n; p += blockDim.x) {
+                const double v = fabs(A[(size_t)order[p] * W.n + k]);
+                const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+                const unsigned long long kv = b <= 0x7ff0000000000000ULL ? b + 1 : 0;
+                if (kv > key) { key = kv; at = p; }
+            }
+            auto take = [&](unsigned long long ok, int oa) {
+                if (ok > key || (ok == key && oa < at)) { key = ok; at = oa; }
+            };
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                take(__shfl_xor_sync(0xffffffffu, key, off), __shfl_xor_sync(0xffffffffu, at, off));
+            if (lane == 0) {
+                best_key[warp] = key;
+                best_at[warp] = at;
+            }
+            __syncthreads();  // also: the order as the last column left it, its readers done
+            key = best_key[0];
+            at = best_at[0];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) take(best_key[q], best_at[q]);
+            const int pr = order[at];
+            const double *P = A + (size_t)pr * W.n;
+            const double diag = P[k];
+            const int kr = order[k];
+            __syncthreads();
+            if (diag == 0.0) {  // the column is skipped, and with it the row at its place
+                if (tid == 0 && kr >= W.lo && kr < W.hi) mine[kr].active = 0;
+            } else {
+                if (tid == 0) {
+                    order[at] = kr;
+                    order[k] = pr;
+                }
+                for (int r = W.lo + warp; r < W.hi; r += 8) {
+                    if (r == pr) {
+                        if (lane == 0) mine[r].active = 0;
+                        continue;
+                    }
+                    if (!mine[r].active) continue;
+                    double *row = A + (size_t)r * W.n;
+                    const double l = row[k] / diag;
+                    if (lane == 0) {
+                        mine[r].l = l;
+                        mine[r].lcol = k;
+                    }
+#pragma unroll 8
+                    for (int c = k + 1 + lane; c < W.n; c += 32) row[c] -= l * P[c];
+                }
+            }
+            __syncthreads();
         }
         grid.sync();
     }
+    for (int i = 0; i < nwin; ++i) {
+        const LuWindow W = wins[i];
+        if (W.lo == 0)
+            for (int p = tid; p < W.n; p += blockDim.x) perm_all[slot_base[W.w] + p] = orders[W.order + p];
+    }
 }
 
+// ordered: perm is the order of the rows, which lie where they were;
+// otherwise the swaps that the rows have been through.
 __global__ void __launch_bounds__(1024) k_wb_lu_solve(const double *Lall, const long long *s_off, const int *n_w,
                                                        const int *slot_base, const int *perm_all, const int *list,
-                                                       const double *rhs, double *x, WinState *ws) {
+                                                       const double *rhs, double *x, WinState *ws, bool ordered) {
     __shared__ double red[32];
     __shared__ int bad;
     const int w = list[blockIdx.x];
@@ -877,10 +951,10 @@ __global__ void __launch_bounds__(1024) k_wb_lu_solve(const double *Lall, const 
     const double *b = rhs + slot_base[w];
     double *xo = x + slot_base[w];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int a = tid; a < n; a += blockDim.x) xo[a] = b[a];
+    for (int a = tid; a < n; a += blockDim.x) xo[a] = b[ordered ? perm[a] : a];
     if (tid == 0) bad = 0;
     __syncthreads();
-    if (tid == 0)
+    if (tid == 0 && !ordered)
         for (int k = 0; k < n; ++k)
             if (perm[k] >= 0 && perm[k] != k) {
                 const double t = xo[k];
@@ -893,19 +967,21 @@ __global__ void __launch_bounds__(1024) k_wb_lu_solve(const double *Lall, const 
         for (int q = 0; q < n; ++q) {
             const int i = pass == 0 ? q : n - 1 - q;
             const int lo = pass == 0 ? 0 : i + 1, hi = pass == 0 ? i : n;
+            const double *row = A + (size_t)(ordered ? perm[i] : i) * n;
             double sum = 0.0;
-            for (int k = lo + tid; k < hi; k += blockDim.x) sum += A[(size_t)i * n + k] * xo[k];
+            for (int k = lo + tid; k < hi; k += blockDim.x) sum += row[k] * xo[k];
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
             if (lane == 0) red[warp] = sum;
             __syncthreads();
             if (tid == 0) {
                 double t = 0.0;
-                for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k];
+                const int used = min((int)(blockDim.x >> 5), (hi - lo + 31) >> 5);  // the other warps' sums are 0
+                for (int k = 0; k < used; ++k) t += red[k];
                 if (pass == 0) {
                     xo[i] -= t;
                 } else {
-                    const double d = A[(size_t)i * n + i];
+                    const double d = row[i];
                     if (d == 0.0) bad = 1;
                     else xo[i] = (xo[i] - t) / d;
                 }
@@ -1153,20 +1229,20 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
     const int nf = n_failed;
     k_wb_lu_copy<<<dim3(64, nf), 256, 0, s>>>(b.S, b.L, w.s_off, w.n_w, w.lu_list);
     SFMBA_LAUNCH_CHECK();
-    static int cap_dev = -1, cap = 0;  // co-resident blocks of the cooperative column loop
-    int dev = 0;
+    // One block per SM: a barrier of more costs more than their warps give.
+    int dev = 0, sms = 0, smem_max = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
-    if (cap_dev != dev) {
-        int per_sm = 0, sms = 0;
-        SFMBA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wb_lu_coop, 256, 0));
-        SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        cap = per_sm * sms;
-        cap_dev = dev;
-    }
-    if (cap > 0) {
+    SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    SFMBA_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const int max_rows = div_up(b.n, sms);
+    const size_t smem = lu_coop_smem(max_rows, w.max_n);
+    const bool ordered = smem + 1024 <= (size_t)smem_max;  // else: a launch per column
+    if (ordered) {
+        SFMBA_CUDA(cudaFuncSetAttribute(k_wb_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)cap);
+        cfg.gridDim = dim3((unsigned)sms);
         cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;
@@ -1174,10 +1250,11 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         SFMBA_CUDA(cudaLaunchKernelEx(&cfg, k_wb_lu_coop, b.L, (const long long *)w.s_off, (const int *)w.n_w,
-                                      (const int *)w.slot_base, b.lu_perm, (const int *)w.lu_list, nf, w.max_n));
+                                      (const int *)w.slot_base, b.lu_perm, (const int *)w.lu_list, nf, w.max_n,
+                                      max_rows));
         SFMBA_LAUNCH_CHECK();
     }
-    for (int k = 0; cap == 0 && k < w.max_n; ++k) {
+    for (int k = 0; !ordered && k < w.max_n; ++k) {
         k_wb_lu_pivot<<<nf, 256, 0, s>>>(b.L, w.s_off, w.n_w, w.slot_base, b.lu_perm, w.lu_list, k);
         SFMBA_LAUNCH_CHECK();
         const int m = w.max_n - k - 1;
@@ -1187,7 +1264,7 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
         SFMBA_LAUNCH_CHECK();
     }
     k_wb_lu_solve<<<nf, 1024, 0, s>>>(b.L, w.s_off, w.n_w, w.slot_base, b.lu_perm, w.lu_list, w.rhs_p, b.work2,
-                                      w.ws);
+                                      w.ws, ordered);
     SFMBA_LAUNCH_CHECK();
 }
 
