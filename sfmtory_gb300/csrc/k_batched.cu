@@ -15,6 +15,7 @@
 #include "camera.cuh"
 #include "chol_block.cuh"
 #include "kernels.cuh"
+#include "lu_rows.cuh"
 #include "ozaki.cuh"
 #include "schur.cuh"
 
@@ -796,144 +797,15 @@ __global__ void k_wb_lu_update(double *Lall, const long long *s_off, const int *
     A[(size_t)r * n + c] -= A[(size_t)r * n + k] * A[(size_t)k * n + c];
 }
 
-// The column loop of the two kernels above in one cooperative launch with one
-// grid barrier per column. The rows of all failed windows are numbered one
-// window after another and dealt to the blocks in runs. No row is swapped:
-// every block keeps the order of the rows of its windows (order[p]: the row at
-// place p), finds the pivot of column k among the places from k on by itself
-// (the first maximum, as above) and updates its own rows that are not pivots
-// yet, a row a warp. A row's multiplier is stored after the next barrier: other
-// blocks may still be searching the column it replaces. Same operations on
-// every entry in the same order, so the same factors; perm receives the order.
-//
-// Bound: the chain of a column (barrier, column, pivot, division, row), not
-// bandwidth: 7.8 ms for one 890-unknown window with its solve, against 13.1 with
-// pivots, swaps and divisions by one block between two barriers.
-struct LuRow {
-    double l;   // multiplier to store ..
-    int lcol;   // .. in this column, -1: none
-    int active; // not a pivot yet
-};
-struct LuWindow {
-    int w, n, order, first, lo, hi;  // its order's place in shared memory; its owned rows lo..hi, first: of the block's
-};
-
-size_t lu_coop_smem(long long rows, int max_n) {
-    return (size_t)rows * (sizeof(LuRow) + sizeof(int)) + (size_t)(rows + 2) * sizeof(LuWindow) +
-           (size_t)2 * max_n * sizeof(int);
-}
-
+// The column loop of the two kernels above in one cooperative launch
+// (lu_rows.cuh); perm receives the order of the rows.
 __global__ void __launch_bounds__(256) k_wb_lu_coop(double *Lall, const long long *s_off, const int *n_w,
                                                      const int *slot_base, int *perm_all, const int *list, int nf,
                                                      int max_n, int max_rows) {
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    extern __shared__ __align__(16) unsigned char lu_sm[];
-    LuRow *rows = reinterpret_cast<LuRow *>(lu_sm);
-    LuWindow *wins = reinterpret_cast<LuWindow *>(rows + max_rows);
-    int *orders = reinterpret_cast<int *>(wins + max_rows + 2);
-    __shared__ unsigned long long best_key[8];
-    __shared__ int best_at[8], nwin;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) {
-        long long total = 0;
-        for (int f = 0; f < nf; ++f) total += n_w[list[f]];
-        const long long per = (total + gridDim.x - 1) / gridDim.x;
-        const long long lo = min(total, per * blockIdx.x), hi = min(total, lo + per);
-        int c = 0, at = 0;
-        long long base = 0;
-        for (int f = 0; f < nf && base < hi; ++f) {
-            const int w = list[f], n = n_w[w];
-            if (n > 0 && base + n > lo) {
-                const int a = (int)(max(lo, base) - base), e = (int)(min(hi, base + n) - base);
-                wins[c++] = {w, n, at, (int)(max(lo, base) - lo), a, e};
-                at += n;
-            }
-            base += n;
-        }
-        nwin = c;
-    }
-    __syncthreads();
-    for (int i = 0; i < nwin; ++i) {
-        const LuWindow W = wins[i];
-        for (int p = tid; p < W.n; p += blockDim.x) orders[W.order + p] = p;
-        for (int r = W.lo + tid; r < W.hi; r += blockDim.x) rows[W.first + r - W.lo] = {0.0, -1, 1};
-    }
-    __syncthreads();
-    for (int k = 0; k <= max_n; ++k) {  // the last turn stores the last multipliers
-        for (int i = 0; i < nwin; ++i) {
-            const LuWindow W = wins[i];
-            if (k > W.n) continue;
-            double *A = Lall + s_off[W.w];
-            LuRow *mine = rows + W.first - W.lo;
-            int *order = orders + W.order;
-            for (int r = W.lo + tid; r < W.hi; r += blockDim.x)
-                if (mine[r].lcol >= 0) {
-                    A[(size_t)r * W.n + mine[r].lcol] = mine[r].l;
-                    mine[r].lcol = -1;
-                }
-            if (k == W.n) continue;
-            // The first maximum: |a| as an integer, 0 for NaN, which no comparison prefers.
-            unsigned long long key = 0;
-            int at = k;
-            for (int p = k + tid; p < W.n; p += blockDim.x) {
-                const double v = fabs(A[(size_t)order[p] * W.n + k]);
-                const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-                const unsigned long long kv = b <= 0x7ff0000000000000ULL ? b + 1 : 0;
-                if (kv > key) { key = kv; at = p; }
-            }
-            auto take = [&](unsigned long long ok, int oa) {
-                if (ok > key || (ok == key && oa < at)) { key = ok; at = oa; }
-            };
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                take(__shfl_xor_sync(0xffffffffu, key, off), __shfl_xor_sync(0xffffffffu, at, off));
-            if (lane == 0) {
-                best_key[warp] = key;
-                best_at[warp] = at;
-            }
-            __syncthreads();  // also: the order as the last column left it, its readers done
-            key = best_key[0];
-            at = best_at[0];
-#pragma unroll
-            for (int q = 1; q < 8; ++q) take(best_key[q], best_at[q]);
-            const int pr = order[at];
-            const double *P = A + (size_t)pr * W.n;
-            const double diag = P[k];
-            const int kr = order[k];
-            __syncthreads();
-            if (diag == 0.0) {  // the column is skipped, and with it the row at its place
-                if (tid == 0 && kr >= W.lo && kr < W.hi) mine[kr].active = 0;
-            } else {
-                if (tid == 0) {
-                    order[at] = kr;
-                    order[k] = pr;
-                }
-                for (int r = W.lo + warp; r < W.hi; r += 8) {
-                    if (r == pr) {
-                        if (lane == 0) mine[r].active = 0;
-                        continue;
-                    }
-                    if (!mine[r].active) continue;
-                    double *row = A + (size_t)r * W.n;
-                    const double l = row[k] / diag;
-                    if (lane == 0) {
-                        mine[r].l = l;
-                        mine[r].lcol = k;
-                    }
-#pragma unroll 8
-                    for (int c = k + 1 + lane; c < W.n; c += 32) row[c] -= l * P[c];
-                }
-            }
-            __syncthreads();
-        }
-        grid.sync();
-    }
-    for (int i = 0; i < nwin; ++i) {
-        const LuWindow W = wins[i];
-        if (W.lo == 0)
-            for (int p = tid; p < W.n; p += blockDim.x) perm_all[slot_base[W.w] + p] = orders[W.order + p];
-    }
+    lu_columns(nf, max_n, max_rows, [&](int f) {
+        const int w = list[f];
+        return LuSystem{Lall + s_off[w], perm_all + slot_base[w], n_w[w]};
+    });
 }
 
 // ordered: perm is the order of the rows, which lie where they were;

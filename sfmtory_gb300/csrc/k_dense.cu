@@ -20,6 +20,7 @@
 
 #include "chol_block.cuh"
 #include "kernels.cuh"
+#include "lu_rows.cuh"
 #include "ozaki.cuh"
 #include "schur.cuh"
 
@@ -341,60 +342,10 @@ __global__ void __launch_bounds__(256) k_chol_update(double *L, int n, int k0, i
 }
 
 // The column loop of k_lu_pivot / k_lu_update (below) in one cooperative
-// launch: block 0 pivots, swaps and scales column k, then every block
-// updates its rows of the trailing matrix; two grid barriers per column
-// instead of two launches, the same operations in the same order (the same
-// factors).
-__global__ void __launch_bounds__(256) k_lu_coop(double *A, int n, int *perm, const LMState *st) {
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    __shared__ double bv[256];
-    __shared__ int bi[256];
+// launch (lu_rows.cuh); perm receives the order of the rows.
+__global__ void __launch_bounds__(256) k_lu_coop(double *A, int n, int *perm, const LMState *st, int max_rows) {
     if (!st->factor_failed || st->solve_failed) return;
-    const int tid = threadIdx.x;
-    for (int k = 0; k < n; ++k) {
-        if (blockIdx.x == 0) {
-            double best = -1.0;
-            int besti = k;
-            for (int r = k + tid; r < n; r += blockDim.x) {
-                const double v = fabs(A[(size_t)r * n + k]);
-                if (v > best) { best = v; besti = r; }
-            }
-            bv[tid] = best;
-            bi[tid] = besti;
-            __syncthreads();
-            for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-                if (tid < h) {
-                    const double o = bv[tid + h];
-                    const int oi = bi[tid + h];
-                    if (o > bv[tid] || (o == bv[tid] && oi < bi[tid])) { bv[tid] = o; bi[tid] = oi; }
-                }
-                __syncthreads();
-            }
-            const int piv = bi[0];
-            const double diag = A[(size_t)piv * n + k];
-            if (diag != 0.0) {
-                if (piv != k)
-                    for (int c = tid; c < n; c += blockDim.x) {
-                        const double t = A[(size_t)k * n + c];
-                        A[(size_t)k * n + c] = A[(size_t)piv * n + c];
-                        A[(size_t)piv * n + c] = t;
-                    }
-                __syncthreads();
-                for (int r = k + 1 + tid; r < n; r += blockDim.x) A[(size_t)r * n + k] /= diag;
-            }
-            if (tid == 0) perm[k] = diag != 0.0 ? piv : -1;  // a zero column is skipped
-            __syncthreads();
-        }
-        grid.sync();
-        if (k + 1 >= n) break;
-        if (((volatile const int *)perm)[k] >= 0)
-            for (int r = k + 1 + blockIdx.x; r < n; r += gridDim.x) {
-                const double lrk = A[(size_t)r * n + k];
-                for (int c = k + 1 + tid; c < n; c += blockDim.x) A[(size_t)r * n + c] -= lrk * A[(size_t)k * n + c];
-            }
-        grid.sync();
-    }
+    lu_columns(1, n, max_rows, [&](int) { return LuSystem{A, perm, n}; });
 }
 
 // ------------------------------------------------ tensor-core trailing update
@@ -631,7 +582,8 @@ __global__ void k_lu_update(double *A, int n, int k, const int *perm, const LMSt
     A[(size_t)r * n + c] -= A[(size_t)r * n + k] * A[(size_t)k * n + c];
 }
 
-// Apply the row swaps to rhs, solve unit-lower then upper. A zero diagonal
+// The rows' order (ordered: they lie where they were) or their swaps applied
+// to rhs, then unit-lower and upper solves. A zero diagonal
 // of U fails the solve (lambda then grows); success clears factor_failed so
 // the back-substitution and trial kernels run.
 // Sum of v over the 1024-thread block (warp sums, then the 32 warps' sums
@@ -649,14 +601,14 @@ __device__ __forceinline__ double block_sum_1024(double v, double *red) {
 }
 
 __global__ void __launch_bounds__(1024) k_lu_solve(const double *A, int n, const int *perm,
-                                                    const double *rhs, double *x, LMState *st) {
+                                                    const double *rhs, double *x, LMState *st, bool ordered) {
     __shared__ double red[32];
     __shared__ int bad;
     if (!st->factor_failed || st->solve_failed) return;
     if (threadIdx.x == 0) bad = 0;
-    for (int a = threadIdx.x; a < n; a += blockDim.x) x[a] = rhs[a];
+    for (int a = threadIdx.x; a < n; a += blockDim.x) x[a] = rhs[ordered ? perm[a] : a];
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && !ordered)
         for (int k = 0; k < n; ++k)
             if (perm[k] >= 0 && perm[k] != k) {
                 const double t = x[k];
@@ -665,18 +617,20 @@ __global__ void __launch_bounds__(1024) k_lu_solve(const double *A, int n, const
             }
     __syncthreads();
     for (int i = 0; i < n; ++i) {
+        const double *row = A + (size_t)(ordered ? perm[i] : i) * n;
         double s = 0.0;
-        for (int k = threadIdx.x; k < i; k += blockDim.x) s += A[(size_t)i * n + k] * x[k];
+        for (int k = threadIdx.x; k < i; k += blockDim.x) s += row[k] * x[k];
         s = block_sum_1024(s, red);
         if (threadIdx.x == 0) x[i] -= s;
         __syncthreads();
     }
     for (int i = n - 1; i >= 0; --i) {
+        const double *row = A + (size_t)(ordered ? perm[i] : i) * n;
         double s = 0.0;
-        for (int k = i + 1 + threadIdx.x; k < n; k += blockDim.x) s += A[(size_t)i * n + k] * x[k];
+        for (int k = i + 1 + threadIdx.x; k < n; k += blockDim.x) s += row[k] * x[k];
         s = block_sum_1024(s, red);
         if (threadIdx.x == 0) {
-            const double d = A[(size_t)i * n + i];
+            const double d = row[i];
             if (d == 0.0) bad = 1;
             else x[i] = (x[i] - s) / d;
         }
@@ -958,21 +912,31 @@ void launch_refine(const Bufs &b, cudaStream_t s) {
     SFMBA_LAUNCH_CHECK();
 }
 
+// Blocks (a row per SM sub-partition, whose FP64 pipe its division and products
+// fill, at most one block per SM) and shared memory of k_lu_coop; false when
+// the rows' order does not fit and the columns take a launch each.
+static bool lu_coop_shape(int n, int &blocks, size_t &smem) {
+    int dev = 0, sms = 0, most = 0;
+    SFMBA_CUDA(cudaGetDevice(&dev));
+    SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    SFMBA_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    blocks = std::min(sms, div_up(n, 4));
+    smem = lu_coop_smem(div_up(n, blocks), n);
+    return smem + 1024 <= (size_t)most;
+}
+
 void launch_lu_factor(const Bufs &b, cudaStream_t s) {
     const int n = b.n;
     SFMBA_CUDA(cudaMemcpyAsync(b.L, b.S, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, s));
-    // One block per SM at most: every column costs two grid barriers, whose
-    // cost grows with the blocks taking part, while its update is small.
-    static int cap_dev = -1, cap = 0, sms = 0;
-    int dev = 0;
-    SFMBA_CUDA(cudaGetDevice(&dev));
-    if (cap_dev != dev) {
-        cap = coop_capacity(k_lu_coop, 0);
-        SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        cap_dev = dev;
-    }
-    if (n > 0 && launch_coop(k_lu_coop, cap, std::min(n, sms), 0, s, b.L, n, b.lu_perm, (const LMState *)b.state))
+    if (n == 0) return;
+    int blocks = 0;
+    size_t smem = 0;
+    if (lu_coop_shape(n, blocks, smem)) {
+        SFMBA_CUDA(cudaFuncSetAttribute(k_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        launch_coop(k_lu_coop, blocks, blocks, smem, s, b.L, n, b.lu_perm, (const LMState *)b.state,
+                    div_up(n, blocks));
         return;
+    }
     for (int k = 0; k < n; ++k) {
         k_lu_pivot<<<1, 1024, 0, s>>>(b.L, n, k, b.lu_perm, b.state);
         SFMBA_LAUNCH_CHECK();
@@ -985,7 +949,10 @@ void launch_lu_factor(const Bufs &b, cudaStream_t s) {
 }
 
 void launch_lu_solve(const Bufs &b, cudaStream_t s) {
-    k_lu_solve<<<1, 1024, 0, s>>>(b.L, b.n, b.lu_perm, b.rhs, b.delta, b.state);
+    int blocks = 0;
+    size_t smem = 0;
+    const bool ordered = b.n > 0 && lu_coop_shape(b.n, blocks, smem);
+    k_lu_solve<<<1, 1024, 0, s>>>(b.L, b.n, b.lu_perm, b.rhs, b.delta, b.state, ordered);
     SFMBA_LAUNCH_CHECK();
 }
 

@@ -1,7 +1,7 @@
 // Throughput probes of the arithmetic units the dense Cholesky can use, the
 // denominators of its roofline: FP64 fused multiply-add (DFMA), the FP64
-// tensor instruction mma.sync m8n8k4 (DMMA) and the BF16 tensor instruction
-// mma.sync m16n8k16 that the error-free split update issues. Each kernel
+// tensor instruction mma.sync m8n8k4 (DMMA) and the warp-level BF16 tensor
+// instruction mma.sync m16n8k16. Each kernel
 // keeps every SM busy with independent dependency chains (enough in flight
 // to cover the unit's latency), is timed with CUDA events after a warm-up
 // launch, and folds its registers into one store that never happens, so
