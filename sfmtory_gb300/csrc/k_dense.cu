@@ -1,8 +1,9 @@
 // Dense reduced camera system:
 //   * Schur reduction S_ij = [i==j] H_i - sum_p E_ip C_p^-1 E_jp^T, one warp
-//     per image pair, walking the pair list grouped by image pair (the
-//     visibility-sorted order), so every block is written exactly once and
-//     no global atomics are used (reference: lib.rs:114-211, :981-1043);
+//     per image pair (FP32) or per chunk of its pairs (FP64, then a sum of the
+//     chunks in order), walking the pair list grouped by image pair (the
+//     visibility-sorted order), so no global atomics are used (reference:
+//     lib.rs:114-211, :981-1043);
 //   * fold of the image-level system onto the reference's slot order with
 //     damping, per-parameter masks and symmetrisation (lib.rs:918-956,
 //     :1051-1074);
