@@ -347,7 +347,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_wb_oz_update(double *Lall, co
     extern __shared__ unsigned char oz_sm[];
     const int w = blockIdx.y;
     const int n = n_w[w];
-    if (!ws[w].active || ws[w].factor_failed) return;
+    // One thread reads the flags (another block may set one): no warp waits for
+    // the tensor memory or the barriers of another that left.
+    if (__syncthreads_or(threadIdx.x == 0 && (!ws[w].active || ws[w].factor_failed))) return;
     int p = blockIdx.x, q = 0;
     for (; p >= (tiles - q + 1) / 2; ++q) p -= (tiles - q + 1) / 2;
     const int rj = k0 + NB + q * kOzCols, ri = rj + p * kOzRows;

@@ -371,7 +371,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_update(double *L, int n, i
                                                              const __nv_bfloat16 *slices, const int *exps,
                                                              LMState *st) {
     extern __shared__ unsigned char oz_sm[];
-    if (st->factor_failed) return;
+    // The next diagonal block may set the flag while this kernel runs: one
+    // thread reads it, so that no warp waits for the tensor memory or the
+    // barriers of another that left.
+    if (__syncthreads_or(threadIdx.x == 0 && st->factor_failed)) return;
     const int c0 = (int)blockIdx.y * NC % 64;
     const int rj = k0 + NB + tj0 * 64 + (int)blockIdx.y * NC, ri = rj - c0 + (int)blockIdx.x * kOzRows;
     if (ri >= n || rj >= n) return;
