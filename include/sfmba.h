@@ -410,6 +410,13 @@ int sfmba_measure_peaks(double *out);
  * SFMBA_ERR_INVALID_ARGUMENT. */
 int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_update, double *seconds);
 
+/* Test aid: sfmba_dense_cholesky with bounded waits that give up at once,
+ * where == 0: for the columns that the blocks of a diagonal block's cluster
+ * send each other, 1: for the slices of the tensor-core tiles. Such a factor is
+ * an SFMBA_ERR_INTERNAL, never "not positive definite"; the kernels end by
+ * themselves and the library stays usable. (L is as undefined as then.) */
+int sfmba_dense_cholesky_give_up(int64_t n, const double *A, double *L, int32_t tensor_update, int32_t where);
+
 /* Benchmarking aid (no counterpart in the reference): when enabled, every
  * kernel phase of the solves made on this thread is bracketed by CUDA events
  * on its launch stream. Enabling or disabling clears the totals. */

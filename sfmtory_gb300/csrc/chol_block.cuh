@@ -50,6 +50,7 @@ struct CholBlock {
 constexpr int kCholCluster = 3;
 
 constexpr int kBlkPolls = 1 << 18;   // bound of every wait for a column
+enum CholStatus { kCholOk = 0, kCholBadPivot = 1, kCholGaveUp = 2 };  // 2: a wait ran out
 constexpr double kBlkFailed = -1.0;  // in place of 1 / L_jj: pivot j or one before it failed
 
 // x < 0 for the marks and reciprocals above, on the integer pipe.
@@ -119,9 +120,9 @@ __device__ __forceinline__ void chol_expect(CholBlock &sm, int first, int second
     }
 }
 
-__device__ __forceinline__ bool chol_wait(const CholBlock &sm, int j) {
+__device__ __forceinline__ bool chol_wait(const CholBlock &sm, int j, int polls) {
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&sm.full[j]);
-    for (int k = 0; k < kBlkPolls; ++k) {
+    for (int k = 0; k < polls; ++k) {
         unsigned ok;
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
@@ -295,8 +296,10 @@ __device__ __forceinline__ int chol_factor_half(double *A, size_t ld, int n, Tri
 }
 
 // Block 1: rows 32.. of the block through block 0's 32 columns as they arrive,
-// then their own factor.
-__device__ __forceinline__ bool chol_rows_behind(double *A, size_t ld, int nb, const CholPeer &inverse, CholBlock &sm) {
+// then their own factor. A wait that gives up ends it as a failed pivot does:
+// block 2 gets a mark for every column, and what block 0 still sends is awaited.
+__device__ __forceinline__ int chol_rows_behind(double *A, size_t ld, int nb, const CholPeer &inverse, CholBlock &sm,
+                                                int polls) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = nb - 32;
     double *A2 = A + 32 * ld + 32;
     TriPatches P(A2, ld, n);
@@ -312,12 +315,12 @@ __device__ __forceinline__ bool chol_rows_behind(double *A, size_t ld, int nb, c
         const int n1 = j + 1;
         const double *L = sm.col + 64 * j;
         if (warp == 0) {
-            const bool ok = __all_sync(0xffffffffu, chol_wait(sm, j));
+            const bool ok = __all_sync(0xffffffffu, chol_wait(sm, j, polls));
             const double inv = ok ? L[j] : kBlkFailed;
             if (is_failed(inv)) {
-                if (lane == 0) sm.failed = 1;
-                for (int i = j; ok && i < nb; ++i) inverse.send(i, 32 + lane, kBlkFailed);
-                for (int i = j + 1; ok && i < 32; ++i) chol_wait(sm, i);  // nothing is under way when the block leaves
+                if (lane == 0) sm.failed = ok ? kCholBadPivot : kCholGaveUp;
+                for (int i = j; i < nb; ++i) inverse.send(i, 32 + lane, kBlkFailed);
+                for (int i = j; i < 32; ++i) chol_wait(sm, i, kBlkPolls);  // nothing is under way when the block leaves
             } else {
                 const double v = sm.raw[lane] * inv;
                 sm.v[lane] = v;
@@ -326,7 +329,7 @@ __device__ __forceinline__ bool chol_rows_behind(double *A, size_t ld, int nb, c
             }
         }
         __syncthreads();
-        if (sm.failed) return false;
+        if (sm.failed) return sm.failed;
         const double v = -sm.v[r];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -339,15 +342,15 @@ __device__ __forceinline__ bool chol_rows_behind(double *A, size_t ld, int nb, c
     }
     const int done = chol_factor_half(A2, ld, n, P, sm, [&](int j, int i, double x) { inverse.send(32 + j, 32 + i, x); });
     for (int i = done; warp == 4 && i < n; ++i) inverse.send(32 + i, 32 + lane, kBlkFailed);
-    return done == n;
+    return done == n ? kCholOk : kCholBadPivot;
 }
 
 // Block 2: X = L^-1 ([64][64], zeros above the diagonal and outside nb), from
 // the columns of L as they arrive. Warp w owns columns 4 w .. 4 w + 3 of
 // either half, a lane the rows congruent to lane / 4 mod 8 of one of them:
 // columns of an inverse do not depend on one another, so the warps meet
-// nowhere. False if a pivot failed or a wait gave up.
-__device__ __forceinline__ bool chol_block_inverse(double *X, int nb, CholBlock &sm) {
+// nowhere. Returns a CholStatus, of the thread's warp.
+__device__ __forceinline__ int chol_block_inverse(double *X, int nb, CholBlock &sm, int polls) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rs = lane >> 2;
     const int c = 4 * w + (lane & 3), d = 32 + c;
     double a[8], b[4];  // rows 8 s + rs of column c, rows 32 + 8 s + rs of column d: minus the sums so far
@@ -356,6 +359,7 @@ __device__ __forceinline__ bool chol_block_inverse(double *X, int nb, CholBlock 
 #pragma unroll
     for (int s = 0; s < 4; ++s) b[s] = 0.0;
     bool ok = true;
+    int status = kCholOk;
 #pragma unroll
     for (int s = 0; s < 8; ++s)
 #pragma unroll
@@ -363,10 +367,13 @@ __device__ __forceinline__ bool chol_block_inverse(double *X, int nb, CholBlock 
             const int j = 8 * s + q;
             double x = 0.0, y = 0.0;
             if (ok && j < nb && j >= 4 * w) {
-                ok = __all_sync(0xffffffffu, chol_wait(sm, j));
+                ok = __all_sync(0xffffffffu, chol_wait(sm, j, polls));
                 const double *L = sm.col + 64 * j;
-                const double inv = L[j];
-                if (is_failed(inv)) ok = false;
+                const double inv = ok ? L[j] : kBlkFailed;
+                if (is_failed(inv)) {
+                    status = ok ? kCholBadPivot : kCholGaveUp;
+                    ok = false;
+                }
                 if (ok) {
                     x = (c == j ? 1.0 : a[s]) * inv;  // row j of X on the lanes of its residue
                     const double xb = __shfl_sync(0xffffffffu, x, 4 * q + (lane & 3));
@@ -385,19 +392,21 @@ __device__ __forceinline__ bool chol_block_inverse(double *X, int nb, CholBlock 
                 X[64 * j + d] = d <= j ? y : 0.0;
             }
         }
-    for (int j = 0; !ok && w == 0 && j < nb; ++j) chol_wait(sm, j);  // nothing is under way when the block leaves
-    return ok;
+    for (int j = 0; !ok && w == 0 && j < nb; ++j) chol_wait(sm, j, kBlkPolls);  // nothing is under way at the end
+    return status;
 }
 
 // The diagonal block at A (row stride ld) by the blocks of a cluster: L below
 // and on the diagonal, its inverse at X. *failed is set when it has none; A
-// and X are then partly written. All blocks call it or none.
-__device__ __forceinline__ void chol_block(double *A, size_t ld, int nb, double *X, CholBlock &sm, int *failed) {
+// and X are then partly written. A wait of more than `polls` attempts gives up:
+// it counts in *timeouts and sets *failed too. All blocks call it or none.
+__device__ __forceinline__ void chol_block(double *A, size_t ld, int nb, double *X, CholBlock &sm, int *failed,
+                                           int *timeouts, int polls) {
     const unsigned rank = cluster_rank();
     const CholPeer rows(sm, 1), inverse(sm, 2);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool both = nb > 32;
-    bool ok = true;
+    int status = kCholOk;
     chol_expect(sm, rank == 2 && both ? 512 : 256, 256);
     if (rank == 0) {
         const int n = min(32, nb);
@@ -408,15 +417,18 @@ __device__ __forceinline__ void chol_block(double *A, size_t ld, int nb, double 
             inverse.send(j, i, x);
         };
         const int done = chol_factor_half(A, ld, n, P, sm, send);
-        ok = done == n;
+        if (done < n) status = kCholBadPivot;
         for (int j = done; warp == 4 && j < n; ++j) send(j, lane, kBlkFailed);
     } else if (rank == 1 && both) {
-        ok = chol_rows_behind(A, ld, nb, inverse, sm);
+        status = chol_rows_behind(A, ld, nb, inverse, sm, polls);
     } else {
         cluster_sync();
-        if (rank == 2) ok = chol_block_inverse(X, nb, sm);
+        if (rank == 2) status = chol_block_inverse(X, nb, sm, polls);
     }
-    if (!ok && lane == 0) *failed = 1;
+    if (status != kCholOk && lane == 0) {
+        *failed = 1;
+        if (status == kCholGaveUp) atomicAdd(timeouts, 1);
+    }
     cluster_sync();  // no block leaves while another sends to it
 }
 

@@ -110,7 +110,9 @@ struct LMState {
     double pcg_tol2;     // stop when |r|^2 <= tol2 |b|^2
     long long pcg_total;  // iterations summed over the whole solve
     int pcg_breakdowns;   // solves ended by p.q <= 0 or r.z <= 0 (not by the tolerance), whole solve
-    int wait_timeouts;    // bounded waits of the TMA point pass that gave up (an internal error)
+    // Bounded waits that gave up (an internal error): of the TMA point pass, the
+    // Cholesky's diagonal blocks and tensor-core tiles, the triangular solves.
+    int wait_timeouts;
 };
 
 #ifdef __CUDACC__

@@ -262,13 +262,14 @@ __global__ void __launch_bounds__(128) k_wb_fold(const int4 *__restrict__ fold_b
 // One cluster of blocks per window.
 __global__ void __cluster_dims__(kCholCluster, 1, 1) __launch_bounds__(256)
     k_wb_chol_diag(double *Lall, const long long *s_off, const int *n_w, double *Linv_all, const long long *linv_off,
-                   int k0, WinState *ws) {
+                   int k0, WinState *ws, LMState *st) {
     __shared__ CholBlock sm;
     const int w = blockIdx.x / kCholCluster;
     const int n = n_w[w];
     if (!ws[w].active || ws[w].factor_failed || k0 >= n) return;
     chol_block(Lall + s_off[w] + (size_t)k0 * n + k0, (size_t)n, min(NB, n - k0),
-               Linv_all + linv_off[w] + (size_t)(k0 / NB) * NB * NB, sm, &ws[w].factor_failed);
+               Linv_all + linv_off[w] + (size_t)(k0 / NB) * NB * NB, sm, &ws[w].factor_failed, &st->wait_timeouts,
+               kBlkPolls);
 }
 
 __global__ void __launch_bounds__(256) k_wb_chol_panel(double *Lall, const long long *s_off, const int *n_w,
@@ -340,15 +341,16 @@ __global__ void __launch_bounds__(256) k_wb_oz_split(const double *Lall, const l
 // of row tiles 2 p and 2 p + 1 below its diagonal tile: block (., w) counts the
 // pairs column by column.
 __global__ void __launch_bounds__(kOzThreads, 1) k_wb_oz_update(double *Lall, const long long *s_off, const int *n_w,
-                                                                int k0, WinState *ws, const int *row_first,
-                                                                const int *slot_base, const long long *linv_off,
+                                                                int k0, const WinState *ws, LMState *st,
+                                                                const int *row_first, const int *slot_base,
+                                                                const long long *linv_off,
                                                                 const __nv_bfloat16 *slices, const int *exps,
                                                                 int tiles) {
     extern __shared__ unsigned char oz_sm[];
     const int w = blockIdx.y;
     const int n = n_w[w];
-    // One thread reads the flags (another block may set one): no warp waits for
-    // the tensor memory or the barriers of another that left.
+    // One thread reads the flags: no warp waits for the tensor memory or the
+    // barriers of another that left.
     if (__syncthreads_or(threadIdx.x == 0 && (!ws[w].active || ws[w].factor_failed))) return;
     int p = blockIdx.x, q = 0;
     for (; p >= (tiles - q + 1) / 2; ++q) p -= (tiles - q + 1) / 2;
@@ -366,8 +368,8 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_wb_oz_update(double *Lall, co
     const __nv_bfloat16 *sl = slices + linv_off[w] / (NB * NB) * kOzBlockElems;
     const bool ok = oz_tile_update<kOzCols>(Lall + s_off[w] + (size_t)ri * n + rj, (size_t)n, mi, mj, p == 0, 0,
                                    sl + (size_t)(ri / 64) * kOzBlockElems, sl + (size_t)(rj / 64) * kOzBlockElems,
-                                   exps + sb + ri, exps + sb + rj, oz_sm);
-    if (!ok && tr == 0) ws[w].factor_failed = 1;  // a wait gave up: the window goes to the LU
+                                   exps + sb + ri, exps + sb + rj, oz_sm, kOzPolls);
+    if (!ok && tr == 0) atomicAdd(&st->wait_timeouts, 1);
 }
 
 // Whole triangular solve L L^T x = b of window w in one CTA (windows are at
@@ -700,7 +702,7 @@ __global__ void k_wb_start_polish(WinState *ws, int W) {
 
 // Batch summary for the host (one block); clears the per-retry accept flags
 // once the commit has consumed them.
-__global__ void __launch_bounds__(256) k_wb_summary(WinState *ws, int W, int *counts) {
+__global__ void __launch_bounds__(256) k_wb_summary(WinState *ws, int W, const LMState *st, int *counts) {
     __shared__ int red[4][256];
     int c[4] = {0, 0, 0, 0};
     for (int w = threadIdx.x; w < W; w += blockDim.x) {
@@ -719,6 +721,7 @@ __global__ void __launch_bounds__(256) k_wb_summary(WinState *ws, int W, int *co
         __syncthreads();
     }
     if (threadIdx.x < 4) counts[threadIdx.x] = red[threadIdx.x][0];
+    if (threadIdx.x == 4) counts[WB_WAIT_TIMEOUTS] = st->wait_timeouts;
 }
 
 // Partial-pivoting LU of the windows whose Cholesky failed (lib.rs:1084-1092),
@@ -982,7 +985,8 @@ void launch_wb_fold(const Bufs &b, const WinBufs &w, cudaStream_t s) {
 void launch_wb_cholesky(const Bufs &b, const WinBufs &w, cudaStream_t s) {
     set_smem_limits();
     for (int k0 = 0; k0 < w.max_n; k0 += NB) {
-        k_wb_chol_diag<<<kCholCluster * w.W, 256, 0, s>>>(b.L, w.s_off, w.n_w, b.Linv, w.linv_off, k0, w.ws);
+        k_wb_chol_diag<<<kCholCluster * w.W, 256, 0, s>>>(b.L, w.s_off, w.n_w, b.Linv, w.linv_off, k0, w.ws,
+                                                          b.state);
         SFMBA_LAUNCH_CHECK();
         const int rem = w.max_n - k0 - NB;
         if (rem <= 0) break;
@@ -998,8 +1002,8 @@ void launch_wb_cholesky(const Bufs &b, const WinBufs &w, cudaStream_t s) {
                                                                     b.oz_exp);
             SFMBA_LAUNCH_CHECK();
             const dim3 gu((unsigned)((tiles + 1) * (tiles + 1) / 4), w.W);
-            k_wb_oz_update<<<gu, kOzThreads, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first, w.slot_base,
-                                                           w.linv_off, (const __nv_bfloat16 *)b.oz_slices, b.oz_exp,
+            k_wb_oz_update<<<gu, kOzThreads, kOzSmem, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, b.state, w.row_first,
+                                                           w.slot_base, w.linv_off, (const __nv_bfloat16 *)b.oz_slices, b.oz_exp,
                                                            (int)tiles);
         } else if (chol_tile(w.W * tiles * (tiles + 1) / 2) == 16) {
             k_wb_chol_update<16><<<grid(div_up(rem, 16)), 256, 0, s>>>(b.L, w.s_off, w.n_w, k0, w.ws, w.row_first,
@@ -1090,8 +1094,8 @@ void launch_wb_start_polish(const WinBufs &w, cudaStream_t s) {
     SFMBA_LAUNCH_CHECK();
 }
 
-void launch_wb_summary(const WinBufs &w, cudaStream_t s) {
-    k_wb_summary<<<1, 256, 0, s>>>(w.ws, w.W, w.counts);
+void launch_wb_summary(const Bufs &b, const WinBufs &w, cudaStream_t s) {
+    k_wb_summary<<<1, 256, 0, s>>>(w.ws, w.W, b.state, w.counts);
     SFMBA_LAUNCH_CHECK();
 }
 

@@ -292,11 +292,11 @@ constexpr int LD = NB + 1;
 // pivot is not > 0 (nalgebra Cholesky::new semantics: 0, negative and NaN all
 // fail).
 __global__ void __cluster_dims__(kCholCluster, 1, 1) __launch_bounds__(256)
-    k_chol_diag(double *L, int n, int k0, double *Linv, LMState *st) {
+    k_chol_diag(double *L, int n, int k0, double *Linv, LMState *st, int polls) {
     __shared__ CholBlock sm;
     if (st->factor_failed) return;
     chol_block(L + (size_t)k0 * n + k0, (size_t)n, min(NB, n - k0), Linv + (size_t)(k0 / NB) * NB * NB, sm,
-               &st->factor_failed);
+               &st->factor_failed, &st->wait_timeouts, polls);
 }
 
 // Panel below the diagonal block k0.
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *L, int n, int k0
 template <int NC>
 __global__ void __launch_bounds__(kOzThreads, 1) k_oz_update(double *L, int n, int k0, int tj0,
                                                              const __nv_bfloat16 *slices, const int *exps,
-                                                             LMState *st) {
+                                                             LMState *st, int polls) {
     extern __shared__ unsigned char oz_sm[];
     // The next diagonal block may set the flag while this kernel runs: one
     // thread reads it, so that no warp waits for the tensor memory or the
@@ -380,8 +380,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_update(double *L, int n, i
     if (ri >= n || rj >= n) return;
     const bool ok = oz_tile_update<NC>(L + (size_t)ri * n + rj, (size_t)n, min(kOzRows, n - ri), min(NC, n - rj),
                                        blockIdx.x == 0, c0, slices + (size_t)(ri / 64) * kOzBlockElems,
-                                       slices + (size_t)(rj / 64) * kOzBlockElems, exps + ri, exps + rj, oz_sm);
-    if (!ok && threadIdx.x == 0) st->factor_failed = 1;  // a wait gave up: the system goes to the LU
+                                       slices + (size_t)(rj / 64) * kOzBlockElems, exps + ri, exps + rj, oz_sm,
+                                       polls);
+    // Not factor_failed: the blocks of k_chol_diag read that beside this kernel and must agree.
+    if (!ok && threadIdx.x == 0) atomicAdd(&st->wait_timeouts, 1);
 }
 
 // Both triangular solves of L L^T x = rhs as a flow of 64-wide blocks over one
@@ -838,11 +840,12 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
     if (n == 0) return;
     const bool oz = b.oz_slices != nullptr;
     const size_t slice_elems = div_up(n, 64) * kOzBlockElems;
+    const int polls = b.give_up_tiles ? 0 : kOzPolls;
     auto slices = [&](int k0) { return (__nv_bfloat16 *)b.oz_slices + ((k0 / NB) & 1) * slice_elems; };
     auto exps = [&](int k0) { return b.oz_exp + ((k0 / NB) & 1) * (size_t)n; };
     // diagonal factor, panel and (tensor path) slices of block k0, on stream st
     auto head = [&](int k0, cudaStream_t st) {
-        k_chol_diag<<<kCholCluster, 256, 0, st>>>(b.L, n, k0, b.Linv, b.state);
+        k_chol_diag<<<kCholCluster, 256, 0, st>>>(b.L, n, k0, b.Linv, b.state, b.give_up_columns ? 0 : kBlkPolls);
         SFMBA_LAUNCH_CHECK();
         const int rem = n - k0 - NB;
         if (rem <= 0) return;
@@ -861,10 +864,10 @@ void launch_cholesky(const Bufs &b, cudaStream_t s) {
             // for n = 2560 against 22).
             if (part == 1)
                 k_oz_update<32><<<dim3(div_up(tiles, 2), 2), kOzThreads, kOzSmem, st>>>(b.L, n, k0, 0, slices(k0),
-                                                                                       exps(k0), b.state);
+                                                                                       exps(k0), b.state, polls);
             else
                 k_oz_update<64><<<dim3(tiles / 2, tiles - 1), kOzThreads, kOzSmem, st>>>(b.L, n, k0, 1, slices(k0),
-                                                                                        exps(k0), b.state);
+                                                                                        exps(k0), b.state, polls);
         } else if (chol_tile(blocks) == 16)
             k_chol_update<16><<<(unsigned)(16 * blocks), 256, 0, st>>>(b.L, n, k0, part, b.state);
         else

@@ -155,6 +155,9 @@ struct Bufs {
     uint16_t *oz_slices = nullptr;
     int *oz_exp = nullptr;
     int *lu_perm = nullptr;       // [n]
+    // Test aid: every wait for a column of a diagonal block, or for a slice of
+    // a tensor-core tile, gives up at once.
+    bool give_up_columns = false, give_up_tiles = false;
     int *trsv_ready = nullptr;    // [2 * blocks of 64] published blocks of the triangular solves (single dense system)
     double *rhs = nullptr, *delta = nullptr, *diagB = nullptr, *work = nullptr, *work2 = nullptr;  // [n]
     double *ref_res = nullptr, *ref_corr = nullptr;  // [n] refinement residual and correction
@@ -235,7 +238,7 @@ struct WinBufs {
     long long *simg_off = nullptr; // [W] offset of its nid_w^2 image-level blocks in S_img
     long long *linv_off = nullptr; // [W] offset of its diagonal-block inverses in Linv
     long long *obs_off = nullptr;  // [W+1] observation range (point-major order)
-    int *counts = nullptr;         // [4] summary read by the host each retry
+    int *counts = nullptr;         // [WB_COUNTS] summary read by the host each retry
     int *slot_perm = nullptr;      // [n] position in the window systems -> slot
     int *row_first = nullptr;      // [n] first nonzero column of each permuted row
     double *rhs_p = nullptr;       // [n] right-hand side in permuted order
@@ -627,7 +630,7 @@ __device__ __forceinline__ void point_inverse_block(const T *pt_C, const T *pt_g
 
 // ---- batched windows (k_batched.cu)
 // Summary counts written by launch_wb_summary.
-enum { WB_NOT_DONE = 0, WB_RETRY_PENDING = 1, WB_FACTOR_FAILED = 2, WB_WANTS_POLISH = 3 };
+enum { WB_NOT_DONE = 0, WB_RETRY_PENDING = 1, WB_FACTOR_FAILED = 2, WB_WANTS_POLISH = 3, WB_WAIT_TIMEOUTS = 4, WB_COUNTS = 5 };
 void launch_wb_window_of_points(const int *win_of_input_point, const int *perm, int nP, int *pt_win,
                                 cudaStream_t s);
 void launch_wb_init(const WinBufs &w, double initial_lambda, cudaStream_t s);
@@ -653,6 +656,6 @@ void launch_wb_reject_failed(const WinBufs &w, cudaStream_t s);
 void launch_wb_end_outer(const WinBufs &w, int max_iterations, bool polish_allowed, double target_cost,
                          cudaStream_t s);
 void launch_wb_start_polish(const WinBufs &w, cudaStream_t s);
-void launch_wb_summary(const WinBufs &w, cudaStream_t s);
+void launch_wb_summary(const Bufs &b, const WinBufs &w, cudaStream_t s);
 
 }  // namespace sfmba

@@ -130,8 +130,8 @@ __device__ __forceinline__ double oz_value(long long L, float T, int x0) {
 
 __device__ __forceinline__ unsigned oz_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool oz_wait(unsigned bar) {
-    for (int k = 0; k < kOzPolls; ++k) {
+__device__ __forceinline__ bool oz_wait(unsigned bar, int polls = kOzPolls) {
+    for (int k = 0; k < polls; ++k) {
         unsigned ok;
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
@@ -171,21 +171,25 @@ __device__ __forceinline__ unsigned long long oz_operand(unsigned at) {
 // the tile is its column c (only c0 + c <= r is written); otherwise c0 is its
 // first column's place in a block of 64. slR / slC: the 64-row blocks of slices
 // of its first rows (the next block follows) and of its columns. eR / eC: the
-// exponents of its rows and columns. smem: kOzSmem bytes. False if a wait gave
-// up.
+// exponents of its rows and columns. smem: kOzSmem bytes. False, and A as it
+// was, if a wait (of `polls` attempts for a slice) gave up; the copies and
+// products under way are awaited all the same.
 template <int NC>
 __device__ __forceinline__ bool oz_tile_update(double *A, size_t lda, int mi, int mj, bool diag, int c0,
                                                const __nv_bfloat16 *slR, const __nv_bfloat16 *slC, const int *eR,
-                                               const int *eC, unsigned char *smem) {
+                                               const int *eC, unsigned char *smem, int polls) {
     constexpr int kWarpCols = NC / 2;
-    __shared__ alignas(8) unsigned long long bars[kOzSlices + 1];  // slice i there; products done
+    // slice i there; products done (tcgen05.commit) and issued (the thread that issues them)
+    __shared__ alignas(8) unsigned long long bars[kOzSlices + 1];
     __shared__ unsigned tmem_at;
+    __shared__ int missed;  // a slice did not come
     __shared__ int xC[NC];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = (oz_smem(smem) + 1023u) & ~1023u, there = oz_smem(&bars[0]), done = oz_smem(&bars[kOzSlices]);
     if (tid == 0) {
         for (int i = 0; i <= kOzSlices; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(there + 8 * i) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(there + 8 * i), "r"(i < kOzSlices ? 1 : 2)
+                         : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         const int halves = mi > 64 ? 2 : 1;
@@ -226,9 +230,10 @@ __device__ __forceinline__ bool oz_tile_update(double *A, size_t lda, int mi, in
         constexpr unsigned kShape = (1u << 4) | (1u << 7) | (1u << 10) | ((NC / 8) << 17) | ((128 / 16) << 24);
         const unsigned cb = diag ? base + c0 * kOzK * 2 : base + kOzColsAt;
         const unsigned col_step = diag ? 2 * kOzSliceBytes : kOzSliceBytes;
-        bool got = oz_wait(there);
+        bool got = true, issued = false;
         for (int d = 2; d <= 8 && got; ++d) {  // weight 2^-8d: slices up to d - 1
-            got = oz_wait(there + 8 * (d - 2));
+            got = oz_wait(there + 8 * (d - 2), polls);
+            issued = issued || got;
             for (int i = max(1, d - kOzSlices); i <= min(kOzSlices, d - 1) && got; ++i)
 #pragma unroll
                 for (int k = 0; k < kOzK / 16; ++k) {
@@ -242,12 +247,16 @@ __device__ __forceinline__ bool oz_tile_update(double *A, size_t lda, int mi, in
                         : "memory");
                 }
         }
-        if (got)
+        missed = !got;
+        if (issued)
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(done)
                          : "memory");
+        else
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(done) : "memory");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(done) : "memory");
     }
     __syncwarp();
-    const bool ok = __all_sync(0xffffffffu, oz_wait(done));
+    const bool over = oz_wait(done), ok = __all_sync(0xffffffffu, over && !missed);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     for (int i = 0; !ok && tid == 0 && i < kOzSlices; ++i) oz_wait(there + 8 * i);  // no copy is under way at the end
     if (ok && __any_sync(0xffffffffu, cols > 0)) {

@@ -345,7 +345,7 @@ Context &context() {
         ctx->device = dev;
         SFMBA_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         SFMBA_CUDA(cudaMallocHost(&ctx->h_state, sizeof(LMState)));
-        SFMBA_CUDA(cudaMallocHost(&ctx->h_counts, 4 * sizeof(int)));
+        SFMBA_CUDA(cudaMallocHost(&ctx->h_counts, WB_COUNTS * sizeof(int)));
     }
     return *ctx;
 }
@@ -1091,7 +1091,7 @@ class Solver {
                 w_.simg_off = A.take<long long>(W);
                 w_.linv_off = A.take<long long>(W);
                 w_.obs_off = A.take<long long>((size_t)W + 1);
-                w_.counts = A.take<int>(4);
+                w_.counts = A.take<int>(WB_COUNTS);
                 w_.slot_perm = A.take<int>(n);
                 const int ncb = (int)batch->cblk_win.size();
                 w_.ncblk = ncb;
@@ -1522,7 +1522,7 @@ class Solver {
                 { SFMBA_PHASE(PH_LM); launch_accept(b, s_); launch_commit(b, s_); }
                 read_state();
                 if (solver_ == SFMBA_SOLVER_DENSE && hs.wait_timeouts)
-                    throw Error(SFMBA_ERR_INTERNAL, "a bounded wait of the triangular solve gave up");
+                    throw Error(SFMBA_ERR_INTERNAL, "a bounded wait of the Cholesky or its triangular solves gave up");
                 if (hs.factor_failed) {
                     // LU fallback on the symmetrised system (lib.rs:1084-1092)
                     { SFMBA_PHASE(PH_LU); launch_lu_factor(b, s_); launch_lu_solve(b, s_); }
@@ -1587,8 +1587,8 @@ class Solver {
         WinBufs &w = w_;
         int *hc = ctx_.h_counts;
         auto counts = [&] {
-            launch_wb_summary(w, s_);
-            SFMBA_CUDA(cudaMemcpyAsync(hc, w.counts, 4 * sizeof(int), cudaMemcpyDeviceToHost, s_));
+            launch_wb_summary(b, w, s_);
+            SFMBA_CUDA(cudaMemcpyAsync(hc, w.counts, WB_COUNTS * sizeof(int), cudaMemcpyDeviceToHost, s_));
             SFMBA_CUDA(cudaStreamSynchronize(s_));
         };
         { SFMBA_PHASE(PH_COST); launch_wb_cost(b, w, false, s_); }
@@ -1646,11 +1646,13 @@ class Solver {
                     { SFMBA_PHASE(PH_BACKSUB); launch_backsub_update(b, b.delta, s_); }
                     { SFMBA_PHASE(PH_COST); launch_wb_cost(b, w, true, s_); }
                     { SFMBA_PHASE(PH_LM); launch_wb_accept_commit(b, w, s_); }
-                    launch_wb_summary(w, s_);
-                    SFMBA_CUDA(cudaMemcpyAsync(hc, w.counts, 4 * sizeof(int), cudaMemcpyDeviceToHost, s_));
+                    launch_wb_summary(b, w, s_);
+                    SFMBA_CUDA(cudaMemcpyAsync(hc, w.counts, WB_COUNTS * sizeof(int), cudaMemcpyDeviceToHost, s_));
                 };
                 retry_round_.run(s_, !profiler().on, round);
                 SFMBA_CUDA(cudaStreamSynchronize(s_));
+                if (hc[WB_WAIT_TIMEOUTS] > 0)  // also set in factor_failed: not the LU's business
+                    throw Error(SFMBA_ERR_INTERNAL, "a bounded wait of the batched Cholesky gave up");
                 if (hc[WB_FACTOR_FAILED] > 0) {
                     // LU fallback for the windows whose Cholesky failed (lib.rs:1084-1092)
                     {
@@ -2765,7 +2767,8 @@ int sfmba_measure_peaks(double *out) {
     });
 }
 
-int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_update, double *seconds) {
+static int dense_cholesky_entry(int64_t n, const double *A, double *L, bool tensor_update, bool give_up_columns,
+                                bool give_up_tiles, double *seconds) {
     return guarded([&] {
         if (n <= 0 || n > 32768) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "n must be in [1, 32768]");
         if (!A || !L) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "A or L is NULL");
@@ -2792,7 +2795,9 @@ int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_u
             b.oz_slices = (uint16_t *)dev_alloc((size_t)2 * div_up((int)n, 64) * kOzBlockElems * sizeof(uint16_t));
             b.oz_exp = (int *)dev_alloc((size_t)2 * n * sizeof(int));
         }
-        int failed = 0;
+        b.give_up_columns = give_up_columns;
+        b.give_up_tiles = give_up_tiles;
+        int failed = 0, timeouts = 0;
         float ms = 0.0f;
         try {
             SFMBA_CUDA(cudaMemcpyAsync(b.L, A, nn * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -2804,6 +2809,7 @@ int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_u
             launch_cholesky(b, s);
             SFMBA_CUDA(cudaEventRecord(e1, s));
             SFMBA_CUDA(cudaMemcpyAsync(&failed, &b.state->factor_failed, sizeof(int), cudaMemcpyDeviceToHost, s));
+            SFMBA_CUDA(cudaMemcpyAsync(&timeouts, &b.state->wait_timeouts, sizeof(int), cudaMemcpyDeviceToHost, s));
             SFMBA_CUDA(cudaMemcpyAsync(L, b.L, nn * sizeof(double), cudaMemcpyDeviceToHost, s));
             SFMBA_CUDA(cudaStreamSynchronize(s));
             SFMBA_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -2814,11 +2820,20 @@ int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_u
             throw;
         }
         for (void *q : owned) cudaFree(q);
+        if (timeouts) throw Error(SFMBA_ERR_INTERNAL, "a bounded wait of the Cholesky gave up");
         if (failed) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "the matrix is not positive definite");
         for (int64_t r = 0; r < n; ++r)
             for (int64_t c = r + 1; c < n; ++c) L[r * n + c] = 0.0;
         if (seconds) *seconds = ms * 1e-3;
     });
+}
+
+int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_update, double *seconds) {
+    return dense_cholesky_entry(n, A, L, tensor_update != 0, false, false, seconds);
+}
+
+int sfmba_dense_cholesky_give_up(int64_t n, const double *A, double *L, int32_t tensor_update, int32_t where) {
+    return dense_cholesky_entry(n, A, L, tensor_update != 0, where == 0, where == 1, nullptr);
 }
 
 const char *sfmba_last_error(void) { return g_last_error.c_str(); }

@@ -49,6 +49,7 @@ EXPORTED_SYMBOLS = (
     "sfmba_total_cost_noalloc",
     "sfmba_measure_peaks",
     "sfmba_dense_cholesky",
+    "sfmba_dense_cholesky_give_up",
     "sfmba_profile_enable",
     "sfmba_profile_report",
     "sfmba_last_error",
@@ -97,6 +98,7 @@ def load(path: str | None = None):
         L.sfmba_local_windows.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32, vp, vp, vp]
         L.sfmba_measure_peaks.argtypes = [vp]
         L.sfmba_dense_cholesky.argtypes = [C.c_int64, vp, vp, C.c_int32, vp]
+        L.sfmba_dense_cholesky_give_up.argtypes = [C.c_int64, vp, vp, C.c_int32, C.c_int32]
         L.sfmba_profile_enable.argtypes = [C.c_int32]
         L.sfmba_profile_report.argtypes = [C.c_char_p, C.c_int64]
         L.sfmba_last_error.restype = C.c_char_p
@@ -413,6 +415,15 @@ def dense_cholesky(A: np.ndarray, tensor_update: bool = True):
     _check(load().sfmba_dense_cholesky(n, A.ctypes.data, L.ctypes.data, 1 if tensor_update else 0,
                                        C.byref(sec)))
     return L, sec.value
+
+
+def dense_cholesky_give_up(A: np.ndarray, tensor_update: bool, tiles: bool) -> None:
+    """The same factor with bounded waits that give up at once (of the tensor-core
+    tiles, else of the diagonal blocks): raises the solver's internal error."""
+    A = np.ascontiguousarray(A, dtype=np.float64)
+    L = np.zeros_like(A)
+    _check(load().sfmba_dense_cholesky_give_up(A.shape[0], A.ctypes.data, L.ctypes.data, 1 if tensor_update else 0,
+                                               1 if tiles else 0))
 
 
 def profile_enable(on: bool = True) -> None:
