@@ -10,18 +10,21 @@
 // The loop ends where rounding decides whether a step lowers the cost, so
 // the order of every sum is part of the result: observation k of a camera
 // belongs to lane k % 128, each lane sums its own in order, and the 128 lane
-// sums are combined in one fixed tree. Within that order the work is spread
-// over the whole GPU: one cooperative kernel takes all cameras through the
-// loop in step. A round is: the terms of every observation (one thread each,
-// the FP64-heavy part), the lane sums (one 128-thread block per camera and
-// quantity, reading the terms), the small solves, and the same two steps for
-// the trial costs. Sums of two products are written as an explicit
-// multiply-add, so that the rounding does not depend on the compiler.
+// sums are combined in one fixed tree. Sums of two products are written as an
+// explicit multiply-add, so that the rounding does not depend on the compiler.
+// Two kernels keep that order, with the same bits:
+//   * few or large cameras: one cooperative kernel takes all cameras through
+//     the loop in step, its work spread over the whole GPU. A round is: the
+//     terms of every observation (one thread each, the FP64-heavy part), the
+//     lane sums (one 128-thread block per camera and quantity, reading the
+//     terms), the small solves, and the same two steps for the trial costs;
+//   * many small cameras: one block per camera for its whole loop, without
+//     terms in memory and without waiting for the other cameras.
 //
 // Bound: the FP64 pipe (17 projections and 16 divisions per observation and
-// iteration). One camera seen in 120 000 observations (OPENCV): 9-12 ms
-// a call against 430-870 ms for one block per camera, which left 151 of 152
-// SMs idle.
+// iteration). One OPENCV camera seen in 120 000 observations: 13 ms a call in
+// step, 640 ms by one block, which leaves 151 of 152 SMs idle. 2000 OPENCV
+// cameras of 400 observations each: 36 ms in step, 18 ms by blocks.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -81,35 +84,43 @@ __device__ __forceinline__ bool obs_residual(const double *poses, const double *
                       ob_xy[2 * (size_t)o + 1], rx, ry);
 }
 
+// Residual r0, weight w and difference columns jx, jy of observation o at
+// `cur`; false for a point behind the camera.
+__device__ __forceinline__ bool obs_columns(const RefineArgs &q, int o, int model, const double *cur, double &r0x,
+                                            double &r0y, double &w, double (&jx)[8], double (&jy)[8]) {
+    const int np = model_dof(model);
+    double pp[8];
+    if (!obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, cur, r0x, r0y)) return false;
+    w = robust_weight<double>(sqrt(__fma_rn(r0x, r0x, __dmul_rn(r0y, r0y))), q.loss, q.scale);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) pp[k] = cur[k];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        jx[a] = jy[a] = 0.0;
+        if (a >= np) continue;
+        double px = r0x, py = r0y, mx = r0x, my = r0y;
+        pp[a] = cur[a] + kFdStep;
+        if (!obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, pp, px, py)) { px = r0x; py = r0y; }
+        pp[a] = cur[a] - kFdStep;
+        if (!obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, pp, mx, my)) { mx = r0x; my = r0y; }
+        pp[a] = cur[a];
+        jx[a] = (px - mx) / (2.0 * kFdStep);
+        jy[a] = (py - my) / (2.0 * kFdStep);
+    }
+    return true;
+}
+
 // Terms of observation o for the normal equations: the products each
 // quantity sums and, last, the weight that multiplies them (all 0 for a
 // point behind the camera or a row's padding, o < 0).
 __device__ __forceinline__ void system_terms(const RefineArgs &q, int o, int model, const double *cur, double *out,
                                              size_t plane) {
     const int np = model_dof(model);
-    double r0x = 0.0, r0y = 0.0, w = 0.0, jx[8], jy[8], pp[8];
-    const bool ok = o >= 0 && obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, cur, r0x, r0y);
-    if (!ok) {
-        r0x = r0y = 0.0;
+    double r0x = 0.0, r0y = 0.0, w = 0.0, jx[8], jy[8];
+    if (o < 0 || !obs_columns(q, o, model, cur, r0x, r0y, w, jx, jy)) {
+        r0x = r0y = w = 0.0;
 #pragma unroll
         for (int a = 0; a < 8; ++a) jx[a] = jy[a] = 0.0;
-    } else {
-        w = robust_weight<double>(sqrt(__fma_rn(r0x, r0x, __dmul_rn(r0y, r0y))), q.loss, q.scale);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) pp[k] = cur[k];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            jx[a] = jy[a] = 0.0;
-            if (a >= np) continue;
-            double px = r0x, py = r0y, mx = r0x, my = r0y;
-            pp[a] = cur[a] + kFdStep;
-            if (!obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, pp, px, py)) { px = r0x; py = r0y; }
-            pp[a] = cur[a] - kFdStep;
-            if (!obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, pp, mx, my)) { mx = r0x; my = r0y; }
-            pp[a] = cur[a];
-            jx[a] = (px - mx) / (2.0 * kFdStep);
-            jy[a] = (py - my) / (2.0 * kFdStep);
-        }
     }
     int e = 0;
 #pragma unroll
@@ -123,21 +134,21 @@ __device__ __forceinline__ void system_terms(const RefineArgs &q, int o, int mod
     out[kRefineSys * plane] = w;
 }
 
-// Terms of observation o for the robust cost w n^2: w n and n.
-__device__ __forceinline__ void cost_terms(const RefineArgs &q, int o, int model, const double *cam, double *out,
-                                           size_t plane) {
-    double wn = 0.0, n = 0.0, rx, ry;
+// Terms of observation o for the robust cost w n^2: w n and n (0 for a point
+// behind the camera or a row's padding).
+__device__ __forceinline__ void cost_terms(const RefineArgs &q, int o, int model, const double *cam, double &wn,
+                                           double &n) {
+    double rx, ry;
+    wn = n = 0.0;
     if (o >= 0 && obs_residual(q.poses, q.points, q.ob_img, q.ob_pt, q.ob_xy, o, model, cam, rx, ry)) {
         n = sqrt(__fma_rn(rx, rx, __dmul_rn(ry, ry)));
         wn = robust_weight<double>(n, q.loss, q.scale) * n;
     }
-    out[0] = wn;
-    out[plane] = n;
 }
 
 // Solves A x = b (n <= 8, row-major, A symmetric): Cholesky, else LU with
 // partial pivoting; false if both fail.
-__device__ bool solve_small(int n, const double *A, const double *b, double *x) {
+__device__ __forceinline__ bool solve_small(int n, const double *A, const double *b, double *x) {
     double L[64];
     bool chol = true;
     for (int j = 0; j < n && chol; ++j) {
@@ -196,6 +207,23 @@ __device__ bool solve_small(int n, const double *A, const double *b, double *x) 
         x[i] = v / M[i * 8 + i];
     }
     return true;
+}
+
+// Trial parameters of a camera: cur plus the step of the system `sys` damped by
+// lambda; cur itself, and false, if it has no solution. One thread.
+__device__ __forceinline__ bool damped_step(const double *sys, int np, double lambda, const double *cur, double *trial) {
+    double A[64], rhs[8], dx[8];
+    int e = 0;
+    for (int a = 0; a < 8; ++a)
+        for (int b = a; b < 8; ++b, ++e)
+            if (a < np && b < np) A[a * np + b] = A[b * np + a] = sys[e];
+    for (int a = 0; a < np; ++a) {
+        rhs[a] = -sys[36 + a];
+        A[a * np + a] += lambda * fmax(A[a * np + a], 1e-12);
+    }
+    const bool solved = solve_small(np, A, rhs, dx);
+    for (int a = 0; a < 8; ++a) trial[a] = cur[a] + (solved && a < np ? dx[a] : 0.0);
+    return solved;
 }
 
 // The lane's running sum over rows [r0, r1) of a chunk: sum of x * y in order
@@ -280,18 +308,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_refine_intrinsics(RefineArgs
             for (int c = blockIdx.x; c < q.nC; c += gridDim.x) {
                 RefineState &s = q.st[c];
                 if (lane != 0 || s.mode == 0) continue;
-                const int np = model_dof(q.cam_model[c]);
-                double A[64], rhs[8], dx[8];
-                int e = 0;
-                for (int a = 0; a < 8; ++a)
-                    for (int b = a; b < 8; ++b, ++e)
-                        if (a < np && b < np) A[a * np + b] = A[b * np + a] = s.sys[e];
-                for (int a = 0; a < np; ++a) {
-                    rhs[a] = -s.sys[36 + a];
-                    A[a * np + a] += s.lambda * fmax(A[a * np + a], 1e-12);
-                }
-                s.solved = solve_small(np, A, rhs, dx) ? 1 : 0;
-                for (int a = 0; a < 8; ++a) s.trial[a] = s.cur[a] + (s.solved && a < np ? dx[a] : 0.0);
+                s.solved = damped_step(s.sys, model_dof(q.cam_model[c]), s.lambda, s.cur, s.trial) ? 1 : 0;
                 s.mode = 2;
                 if (!s.solved) {  // intrinsics.rs:202-205
                     s.lambda *= 3.0;
@@ -309,8 +326,8 @@ __global__ void __launch_bounds__(kRefineThreads) k_refine_intrinsics(RefineArgs
                 const int c = q.row_cam[row];
                 const RefineState &s = q.st[c];
                 if (s.mode == 0 || !s.solved) continue;
-                cost_terms(q, q.row_obs[(size_t)row * kRefineLanes + lane], q.cam_model[c], s.trial,
-                           q.terms + (size_t)(row - lo) * kRefineLanes + lane, plane);
+                double *out = q.terms + (size_t)(row - lo) * kRefineLanes + lane;
+                cost_terms(q, q.row_obs[(size_t)row * kRefineLanes + lane], q.cam_model[c], s.trial, out[0], out[plane]);
             }
             grid.sync();
             const int c0 = q.row_cam[lo], c1 = q.row_cam[hi - 1];
@@ -359,7 +376,94 @@ __global__ void __launch_bounds__(kRefineThreads) k_refine_intrinsics(RefineArgs
         if (lane < 8) q.cams[8 * (size_t)c + lane] = q.st[c].cur[lane];
 }
 
+// Robust cost of the parameters `cam` over rows [r0, r1), by the block.
+__device__ double block_cost(const RefineArgs &q, int r0, int r1, int model, const double *cam, double *sh) {
+    double sum = 0.0;
+    for (int r = r0; r < r1; ++r) {
+        double wn, n;
+        cost_terms(q, q.row_obs[(size_t)r * kRefineLanes + threadIdx.x], model, cam, wn, n);
+        sum = fma(wn, n, sum);
+    }
+    return block_sum128(sum, sh);
+}
+
+// One block per camera for its whole loop.
+__global__ void __launch_bounds__(kRefineThreads) k_refine_cameras(RefineArgs q) {
+    __shared__ double sh[4], cur[8], trial[8], sys[kRefineSys];
+    __shared__ int solved;
+    const int c = blockIdx.x, lane = threadIdx.x, r0 = q.cam_row0[c], r1 = q.cam_row0[c + 1];
+    if (r0 == r1) return;  // intrinsics.rs:135-141: left as it is
+    const int model = q.cam_model[c], np = model_dof(model);
+    if (lane < 8) cur[lane] = q.cams[8 * (size_t)c + lane];
+    __syncthreads();
+    double cost = block_cost(q, r0, r1, model, cur, sh), lambda = q.lambda0;
+    for (int it = 0; it < q.max_iterations; ++it) {
+        double acc[kRefineSys];
+#pragma unroll
+        for (int e = 0; e < kRefineSys; ++e) acc[e] = 0.0;
+        for (int r = r0; r < r1; ++r) {
+            const int o = q.row_obs[(size_t)r * kRefineLanes + lane];
+            double r0x, r0y, w, jx[8], jy[8];
+            if (o < 0 || !obs_columns(q, o, model, cur, r0x, r0y, w, jx, jy)) continue;
+            int e = 0;
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+#pragma unroll
+                for (int b = a; b < 8; ++b, ++e)
+                    if (b < np) acc[e] = fma(w, __fma_rn(jx[a], jx[b], __dmul_rn(jy[a], jy[b])), acc[e]);
+#pragma unroll
+            for (int a = 0; a < 8; ++a, ++e)
+                if (a < np) acc[e] = fma(w, __fma_rn(jx[a], r0x, __dmul_rn(jy[a], r0y)), acc[e]);
+        }
+        auto total = [&](int e, double v) {
+            v = block_sum128(v, sh);
+            if (lane == 0) sys[e] = v;
+        };
+        int e = 0;
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+            for (int b = a; b < 8; ++b, ++e)
+                if (b < np) total(e, acc[e]);
+#pragma unroll
+        for (int a = 0; a < 8; ++a, ++e)
+            if (a < np) total(e, acc[e]);
+        __syncthreads();
+        bool accepted = false;
+        for (int t = 0; t < 8; ++t) {
+            if (lane == 0) solved = damped_step(sys, np, lambda, cur, trial);
+            __syncthreads();
+            if (solved) {
+                const double tc = block_cost(q, r0, r1, model, trial, sh);
+                if (isfinite(tc) && tc < cost) {
+                    cost = tc;
+                    accepted = true;
+                    break;
+                }
+            }
+            lambda *= 3.0;  // intrinsics.rs:202-205, for a system without a solution too
+            __syncthreads();
+        }
+        if (!accepted) break;
+        lambda = fmax(lambda / 3.0, 1e-12);
+        if (lane < 8) cur[lane] = trial[lane];
+        __syncthreads();
+    }
+    if (lane < 8) q.cams[8 * (size_t)c + lane] = cur[lane];
+}
+
 }  // namespace
+
+// In step or a block per camera. In step pays for its barriers and for the
+// (camera, quantity) sums of every round, a block for the rows of the largest
+// camera, one after another. Measured, block time / time in step (SIMPLE_RADIAL,
+// OPENCV alike): 1 camera of 1, 2, 4, 16 rows 0.98, 1.1, 1.7, 3.9; 50 cameras of
+// 2, 4, 8, 32 rows 0.7, 1.05, 1.5, 2.9; 150 of 4, 8, 32 rows 0.8, 1.1, 1.2; 300 of
+// 4 to 16 rows 0.7 to 0.9, however many rows: then the blocks fill the GPU, so
+// the largest camera has to hold more than 3/5 of an SM's share of all rows.
+bool refine_in_step(int cameras, int most_rows, int rows, int sms) {
+    return cameras + 45LL <= 25LL * most_rows && 3LL * rows <= 5LL * most_rows * sms;
+}
 
 size_t refine_state_bytes() { return sizeof(RefineState); }
 
@@ -374,6 +478,11 @@ void launch_refine_intrinsics(const IntrinsicsBufs &q, int max_iterations, doubl
     a.cams = q.cams;
     a.nC = q.nC; a.rows = q.rows; a.chunk_rows = std::min(q.rows, kRefineChunkRows);
     a.max_iterations = max_iterations; a.loss = loss; a.lambda0 = lambda0; a.scale = scale;
+    if (!q.in_step) {
+        k_refine_cameras<<<q.nC, kRefineThreads, 0, s>>>(a);
+        SFMBA_LAUNCH_CHECK();
+        return;
+    }
     int dev = 0, per_sm = 0, sms = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     SFMBA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_refine_intrinsics, kRefineThreads, 0));

@@ -428,8 +428,9 @@ struct IntrinsicsBufs {
     const double *poses = nullptr, *points = nullptr, *ob_xy = nullptr;
     const int *ob_img = nullptr, *ob_pt = nullptr, *cam_model = nullptr;
     // Observations grouped by camera in rows of kRefineLanes (cameras with
-    // fewer than 8 have none), and the kernel's work space.
+    // fewer than 8 have none), and the work space of the cameras in step.
     int rows = 0;
+    bool in_step = false;  // refine_in_step
     const int *row_cam = nullptr, *cam_row0 = nullptr, *row_obs = nullptr;
     double *terms = nullptr;                 // [kRefineTerms][min(rows, kRefineChunkRows)][kRefineLanes]
     double *lane_sum = nullptr;              // [2][kRefineTerms - 1][kRefineLanes]
@@ -440,6 +441,7 @@ struct IntrinsicsBufs {
 constexpr int kRefineLanes = 128;       // lanes an observation sum is split into
 constexpr int kRefineTerms = 45;        // 44 sums and the weight
 constexpr int kRefineChunkRows = 2048;  // rows whose terms are held at once (94 MB, below the L2)
+bool refine_in_step(int cameras, int most_rows, int rows, int sms);
 size_t refine_state_bytes();
 void launch_refine_intrinsics(const IntrinsicsBufs &q, int max_iterations, double lambda0, int loss, double scale,
                               cudaStream_t s);

@@ -2585,10 +2585,11 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
         // order, in rows of kRefineLanes; cameras with fewer than 8 have none.
         std::vector<int> count(nC, 0), row0(nC + 1, 0), row_cam;
         for (long long k = 0; k < nO; ++k) count[p->camera_of_image[p->obs_image[k]]] += 1;
-        int active = 0;
+        int active = 0, most_rows = 0;
         for (int c = 0; c < nC; ++c) {
             const int rows = count[c] >= 8 ? div_up(count[c], kRefineLanes) : 0;
             active += rows > 0;
+            most_rows = std::max(most_rows, rows);
             row0[c + 1] = row0[c] + rows;
             row_cam.insert(row_cam.end(), rows, c);
         }
@@ -2604,6 +2605,9 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
         }
         Arena &A = ctx.aux;
         IntrinsicsBufs q;
+        int sms = 0;
+        SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+        q.in_step = refine_in_step(active, most_rows, rows, sms);
         double *poses = nullptr, *points = nullptr, *xy = nullptr, *cam = nullptr;
         int *img = nullptr, *pt = nullptr, *model = nullptr, *d_row_cam = nullptr, *d_row0 = nullptr, *d_row_obs = nullptr;
         for (int pass = 0; pass < 2; ++pass) {
@@ -2618,6 +2622,7 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
             d_row_cam = A.take<int>(rows);
             d_row0 = A.take<int>((size_t)nC + 1);
             d_row_obs = A.take<int>(row_obs.size());
+            if (!q.in_step) continue;
             q.terms = A.take<double>((size_t)kRefineTerms * std::min(rows, kRefineChunkRows) * kRefineLanes);
             q.lane_sum = A.take<double>((size_t)2 * (kRefineTerms - 1) * kRefineLanes);
             q.state = A.take<char>((size_t)nC * refine_state_bytes());
@@ -2633,7 +2638,7 @@ int sfmba_refine_intrinsics(const sfmba_problem *p, const sfmba_options *o, doub
         put_vec(d_row_cam, row_cam, s);
         put_vec(d_row0, row0, s);
         put_vec(d_row_obs, row_obs, s);
-        put(q.active, &active, 1, false, s);
+        if (q.in_step) put(q.active, &active, 1, false, s);
         q.nC = nC; q.poses = poses; q.points = points; q.ob_xy = xy; q.ob_img = img; q.ob_pt = pt;
         q.cam_model = model; q.rows = rows; q.row_cam = d_row_cam; q.cam_row0 = d_row0; q.row_obs = d_row_obs;
         q.cams = cam;
