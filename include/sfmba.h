@@ -417,6 +417,16 @@ int sfmba_dense_cholesky(int64_t n, const double *A, double *L, int32_t tensor_u
  * themselves and the library stays usable. (L is as undefined as then.) */
 int sfmba_dense_cholesky_give_up(int64_t n, const double *A, double *L, int32_t tensor_update, int32_t where);
 
+/* Test aid (lib.rs:1084-1092 on its own): the LU that the solves fall back to
+ * where a Cholesky fails, applied to `num` square systems A_k x_k = b_k (host;
+ * n[k] unknowns, A_k row-major, all one after another). batched == 0: the dense
+ * solver's kernels (num must be 1), else those of the batched solves.
+ * by_columns != 0: the form of a launch per column, which the solves take for
+ * systems too large for the one-launch form. solved[k]: 0 where U has a zero on
+ * its diagonal; x_k is then undefined. */
+int sfmba_dense_lu(int32_t num, const int64_t *n, const double *A, const double *b, double *x, int32_t batched,
+                   int32_t by_columns, int32_t *solved);
+
 /* Benchmarking aid (no counterpart in the reference): when enabled, every
  * kernel phase of the solves made on this thread is bracketed by CUDA events
  * on its launch stream. Enabling or disabling clears the totals. */

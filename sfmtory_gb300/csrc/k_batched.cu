@@ -1114,7 +1114,7 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
     SFMBA_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const int max_rows = div_up(b.n, sms);
     const size_t smem = lu_coop_smem(max_rows, w.max_n);
-    const bool ordered = smem + 1024 <= (size_t)smem_max;  // else: a launch per column
+    const bool ordered = !b.lu_by_columns && smem + 1024 <= (size_t)smem_max;  // else: a launch per column
     if (ordered) {
         SFMBA_CUDA(cudaFuncSetAttribute(k_wb_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         cudaLaunchConfig_t cfg{};

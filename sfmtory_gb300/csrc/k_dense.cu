@@ -938,7 +938,7 @@ void launch_lu_factor(const Bufs &b, cudaStream_t s) {
     if (n == 0) return;
     int blocks = 0;
     size_t smem = 0;
-    if (lu_coop_shape(n, blocks, smem)) {
+    if (!b.lu_by_columns && lu_coop_shape(n, blocks, smem)) {
         SFMBA_CUDA(cudaFuncSetAttribute(k_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         launch_coop(k_lu_coop, blocks, blocks, smem, s, b.L, n, b.lu_perm, (const LMState *)b.state,
                     div_up(n, blocks));
@@ -958,7 +958,7 @@ void launch_lu_factor(const Bufs &b, cudaStream_t s) {
 void launch_lu_solve(const Bufs &b, cudaStream_t s) {
     int blocks = 0;
     size_t smem = 0;
-    const bool ordered = b.n > 0 && lu_coop_shape(b.n, blocks, smem);
+    const bool ordered = !b.lu_by_columns && b.n > 0 && lu_coop_shape(b.n, blocks, smem);
     k_lu_solve<<<1, 1024, 0, s>>>(b.L, b.n, b.lu_perm, b.rhs, b.delta, b.state, ordered);
     SFMBA_LAUNCH_CHECK();
 }

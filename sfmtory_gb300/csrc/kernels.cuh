@@ -158,6 +158,7 @@ struct Bufs {
     // Test aid: every wait for a column of a diagonal block, or for a slice of
     // a tensor-core tile, gives up at once.
     bool give_up_columns = false, give_up_tiles = false;
+    bool lu_by_columns = false;  // test aid: the LU's form of a launch per column, whatever the size
     int *trsv_ready = nullptr;    // [2 * blocks of 64] published blocks of the triangular solves (single dense system)
     double *rhs = nullptr, *delta = nullptr, *diagB = nullptr, *work = nullptr, *work2 = nullptr;  // [n]
     double *ref_res = nullptr, *ref_corr = nullptr;  // [n] refinement residual and correction

@@ -2841,6 +2841,78 @@ int sfmba_dense_cholesky_give_up(int64_t n, const double *A, double *L, int32_t 
     return dense_cholesky_entry(n, A, L, tensor_update != 0, where == 0, where == 1, nullptr);
 }
 
+int sfmba_dense_lu(int32_t num, const int64_t *n, const double *A, const double *b, double *x, int32_t batched,
+                   int32_t by_columns, int32_t *solved) {
+    return guarded([&] {
+        if (num <= 0 || (!batched && num != 1)) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "wrong number of systems");
+        if (!n || !A || !b || !x || !solved) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "an argument is NULL");
+        std::vector<int> n_w(num), slot_base(num);
+        std::vector<long long> s_off(num);
+        long long slots = 0, entries = 0;
+        WinBufs w;
+        for (int k = 0; k < num; ++k) {
+            if (n[k] <= 0 || n[k] > 32768) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "n must be in [1, 32768]");
+            n_w[k] = (int)n[k];
+            slot_base[k] = (int)slots;
+            s_off[k] = entries;
+            slots += n[k];
+            entries += n[k] * n[k];
+            w.max_n = std::max(w.max_n, n_w[k]);
+        }
+        if (slots > INT_MAX) throw Error(SFMBA_ERR_INVALID_ARGUMENT, "too many unknowns");
+        Context &ctx = context();
+        cudaStream_t s = ctx.stream;
+        Arena &M = ctx.aux;
+        Bufs d;
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 0) M.begin_sizing(); else M.commit();
+            d.S = M.take<double>(entries);
+            d.L = M.take<double>(entries);
+            d.lu_perm = M.take<int>(slots);
+            d.rhs = M.take<double>(slots);
+            d.delta = M.take<double>(slots);
+            d.state = M.take<LMState>(1);
+            w.ws = M.take<WinState>(num);
+            w.n_w = M.take<int>(num);
+            w.slot_base = M.take<int>(num);
+            w.s_off = M.take<long long>(num);
+            w.lu_list = M.take<int>(num);
+            w.lu_count = M.take<int>(1);
+        }
+        d.n = (int)slots;
+        d.work2 = d.delta;
+        d.lu_by_columns = by_columns != 0;
+        w.W = num;
+        w.rhs_p = d.rhs;
+        LMState st{};
+        st.factor_failed = 1;
+        std::vector<WinState> ws(num);
+        for (WinState &v : ws) {
+            v = WinState{};
+            v.active = v.factor_failed = 1;
+        }
+        put(d.S, A, (size_t)entries, false, s);
+        put(d.rhs, b, (size_t)slots, false, s);
+        put(d.state, &st, 1, false, s);
+        put_vec(w.ws, ws, s);
+        put_vec(w.n_w, n_w, s);
+        put_vec(w.slot_base, slot_base, s);
+        put_vec(w.s_off, s_off, s);
+        SFMBA_CUDA(cudaMemsetAsync(d.delta, 0, sizeof(double) * (size_t)slots, s));
+        if (batched) {
+            launch_wb_lu(d, w, num, s);
+        } else {
+            launch_lu_factor(d, s);
+            launch_lu_solve(d, s);
+        }
+        SFMBA_CUDA(cudaMemcpyAsync(x, d.delta, sizeof(double) * (size_t)slots, cudaMemcpyDeviceToHost, s));
+        SFMBA_CUDA(cudaMemcpyAsync(&st, d.state, sizeof(LMState), cudaMemcpyDeviceToHost, s));
+        SFMBA_CUDA(cudaMemcpyAsync(ws.data(), w.ws, sizeof(WinState) * (size_t)num, cudaMemcpyDeviceToHost, s));
+        SFMBA_CUDA(cudaStreamSynchronize(s));
+        for (int k = 0; k < num; ++k) solved[k] = batched ? !ws[k].factor_failed : !st.factor_failed;
+    });
+}
+
 const char *sfmba_last_error(void) { return g_last_error.c_str(); }
 
 const char *sfmba_version(void) { return "sfmba-gb300 0.1 (sm_103a)"; }

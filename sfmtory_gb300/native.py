@@ -50,6 +50,7 @@ EXPORTED_SYMBOLS = (
     "sfmba_measure_peaks",
     "sfmba_dense_cholesky",
     "sfmba_dense_cholesky_give_up",
+    "sfmba_dense_lu",
     "sfmba_profile_enable",
     "sfmba_profile_report",
     "sfmba_last_error",
@@ -98,6 +99,7 @@ def load(path: str | None = None):
         L.sfmba_local_windows.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32, vp, vp, vp]
         L.sfmba_measure_peaks.argtypes = [vp]
         L.sfmba_dense_cholesky.argtypes = [C.c_int64, vp, vp, C.c_int32, vp]
+        L.sfmba_dense_lu.argtypes = [C.c_int32, vp, vp, vp, vp, C.c_int32, C.c_int32, vp]
         L.sfmba_dense_cholesky_give_up.argtypes = [C.c_int64, vp, vp, C.c_int32, C.c_int32]
         L.sfmba_profile_enable.argtypes = [C.c_int32]
         L.sfmba_profile_report.argtypes = [C.c_char_p, C.c_int64]
@@ -424,6 +426,20 @@ def dense_cholesky_give_up(A: np.ndarray, tensor_update: bool, tiles: bool) -> N
     L = np.zeros_like(A)
     _check(load().sfmba_dense_cholesky_give_up(A.shape[0], A.ctypes.data, L.ctypes.data, 1 if tensor_update else 0,
                                                1 if tiles else 0))
+
+
+def dense_lu(matrices, rhs, batched: bool = True, by_columns: bool = False):
+    """The LU fallback of the dense (one system) or the batched solver on
+    ``matrices`` x = ``rhs``: a list of solutions, None for a singular system."""
+    n = np.array([len(b) for b in rhs], np.int64)
+    A = np.concatenate([np.asarray(m, np.float64).reshape(-1) for m in matrices])
+    b = np.concatenate([np.asarray(v, np.float64).reshape(-1) for v in rhs])
+    if len(A) != int((n * n).sum()):
+        raise ValueError("one square matrix per right-hand side")
+    x, solved = np.zeros_like(b), np.zeros(len(n), np.int32)
+    _check(load().sfmba_dense_lu(len(n), n.ctypes.data, A.ctypes.data, b.ctypes.data, x.ctypes.data,
+                                 1 if batched else 0, 1 if by_columns else 0, solved.ctypes.data))
+    return [v if ok else None for v, ok in zip(np.split(x, np.cumsum(n)[:-1]), solved)]
 
 
 def profile_enable(on: bool = True) -> None:
