@@ -1107,18 +1107,37 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
     const int nf = n_failed;
     k_wb_lu_copy<<<dim3(64, nf), 256, 0, s>>>(b.S, b.L, w.s_off, w.n_w, w.lu_list);
     SFMBA_LAUNCH_CHECK();
-    // One block per SM: a barrier of more costs more than their warps give.
     int dev = 0, sms = 0, smem_max = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     SFMBA_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const int max_rows = div_up(b.n, sms);
-    const size_t smem = lu_coop_smem(max_rows, w.max_n);
-    const bool ordered = !b.lu_by_columns && smem + 1024 <= (size_t)smem_max;  // else: a launch per column
-    if (ordered) {
-        SFMBA_CUDA(cudaFuncSetAttribute(k_wb_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The windows that one launch takes: those whose rows' order fits in the
+    // blocks' shared memory (3900 windows of 200 unknowns, 770 of 1000).
+    const long long fit = ((long long)smem_max - 1024 - (long long)lu_coop_smem(0, w.max_n)) /
+                          (long long)(lu_coop_smem(1, 0) - lu_coop_smem(0, 0));
+    const int group = (int)std::min<long long>(nf, fit * sms / w.max_n);
+    const bool ordered = !b.lu_by_columns && group > 0;  // else: a launch per column
+    for (int f = 0; ordered && f < nf; f += group) {
+        const int m = std::min(group, nf - f);
+        const long long unknowns = std::min<long long>(b.n, (long long)m * w.max_n);
+        // Blocks per SM: one window is a chain of columns, which more blocks only
+        // lengthen at the barrier (833 unknowns: 8.7 ms with one, 9.0 with four).
+        // Several windows are work for more warps: four blocks against one take
+        // 9.7 against 13.0 ms for 2 of 833, 79 against 154 for 64, 32 against 50
+        // for 512 of 273, 27 against 36 for 2000 of 133.
+        int per_sm = m > 1 ? 4 : 1, max_rows = 0;
+        size_t smem = 0;
+        for (;; --per_sm) {
+            max_rows = div_up(unknowns, (long long)per_sm * sms);
+            smem = lu_coop_smem(max_rows, w.max_n);
+            SFMBA_CUDA(cudaFuncSetAttribute(k_wb_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            int resident = 0;
+            SFMBA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_wb_lu_coop, 256, smem));
+            if (resident >= per_sm) break;
+            if (per_sm == 1) throw Error(SFMBA_ERR_INTERNAL, "the batch's LU does not fit the GPU");
+        }
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)sms);
+        cfg.gridDim = dim3((unsigned)(per_sm * sms));
         cfg.blockDim = dim3(256);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
@@ -1128,7 +1147,7 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         SFMBA_CUDA(cudaLaunchKernelEx(&cfg, k_wb_lu_coop, b.L, (const long long *)w.s_off, (const int *)w.n_w,
-                                      (const int *)w.slot_base, b.lu_perm, (const int *)w.lu_list, nf, w.max_n,
+                                      (const int *)w.slot_base, b.lu_perm, (const int *)(w.lu_list + f), m, w.max_n,
                                       max_rows));
         SFMBA_LAUNCH_CHECK();
     }

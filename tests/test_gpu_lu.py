@@ -68,7 +68,8 @@ def test_one_system(kind, n, batched):
 
 
 @pytest.mark.parametrize("sizes", [(1, 1), (333, 1, 7, 64, 40), (200, 201, 199, 3), tuple(range(1, 60)) * 3,
-                                   (24,) * 700, (300,) * 24], ids=["ones", "unequal", "large", "many", "small", "shared"])
+                                   (24,) * 700, (300,) * 24, (2000,) + (2, 3) * 500],
+                         ids=["ones", "unequal", "large", "many", "small", "shared", "several_launches"])
 def test_windows_of_a_batch(sizes):
     rng = np.random.default_rng(len(sizes))
     As = [_matrix(KINDS[k % len(KINDS)], n, rng) for k, n in enumerate(sizes)]
