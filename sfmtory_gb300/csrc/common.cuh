@@ -39,6 +39,20 @@ extern thread_local long long g_kernel_launches;
         SFMBA_CUDA(cudaGetLastError());     \
     } while (0)
 
+// Lets launches of kernel k have all the shared memory of a block beside its
+// static part, on the current device. The limit belongs to the function, not to
+// the launch: set to one launch's need it would be lowered by another host
+// thread before that launch. The same value always, so any thread may set it.
+template <typename K>
+void allow_shared_memory(K k) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes a;
+    SFMBA_CUDA(cudaGetDevice(&dev));
+    SFMBA_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    SFMBA_CUDA(cudaFuncGetAttributes(&a, k));
+    SFMBA_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+}
+
 constexpr int kMaxParams = SFMBA_MAX_CAMERA_PARAMS;
 constexpr double kMinDepth = 1e-9;            // crates/sfm-ba/src/lib.rs:256, 338
 constexpr double kFunctionTolerance = 1e-6;   // lib.rs:814

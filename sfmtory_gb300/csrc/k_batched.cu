@@ -887,10 +887,13 @@ void dispatch_D(int D, F &&f) {
 
 
 void set_smem_limits() {
-    static bool done = false;
-    if (done) return;
-    SFMBA_CUDA(cudaFuncSetAttribute(k_wb_oz_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
-    done = true;
+    thread_local int done_dev = -1;
+    int dev = 0;
+    SFMBA_CUDA(cudaGetDevice(&dev));
+    if (done_dev == dev) return;
+    allow_shared_memory(k_wb_oz_update);
+    allow_shared_memory(k_wb_lu_coop);
+    done_dev = dev;
 }
 
 int grid1(int n) { return div_up(n > 0 ? n : 1, 128); }
@@ -1107,6 +1110,7 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
     const int nf = n_failed;
     k_wb_lu_copy<<<dim3(64, nf), 256, 0, s>>>(b.S, b.L, w.s_off, w.n_w, w.lu_list);
     SFMBA_LAUNCH_CHECK();
+    set_smem_limits();
     int dev = 0, sms = 0, smem_max = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1130,7 +1134,6 @@ void launch_wb_lu(const Bufs &b, const WinBufs &w, int n_failed, cudaStream_t s)
         for (;; --per_sm) {
             max_rows = div_up(unknowns, (long long)per_sm * sms);
             smem = lu_coop_smem(max_rows, w.max_n);
-            SFMBA_CUDA(cudaFuncSetAttribute(k_wb_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int resident = 0;
             SFMBA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_wb_lu_coop, 256, smem));
             if (resident >= per_sm) break;

@@ -723,7 +723,7 @@ void launch_coarse_invert(const Bufs &b, cudaStream_t s) {
     const CoarseBufs &co = b.co;
     const int Nc = co.nc * b.D, Np = coarse_padded_size(Nc);
     SFMBA_CUDA(cudaMemsetAsync(co.fail, 0, 2 * sizeof(int), s));
-    static int cap_dev = -1, cap = 0;  // co-resident blocks, queried once per device
+    thread_local int cap_dev = -1, cap = 0;  // co-resident blocks, queried once per thread and device
     int dev = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     if (cap_dev != dev) {

@@ -663,11 +663,14 @@ void dispatch_D(int D, F &&f) {
 
 
 void set_smem_limits() {
-    static bool done = false;
-    if (done) return;
-    SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
-    SFMBA_CUDA(cudaFuncSetAttribute(k_oz_update<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
-    done = true;
+    thread_local int done_dev = -1;
+    int dev = 0;
+    SFMBA_CUDA(cudaGetDevice(&dev));
+    if (done_dev == dev) return;
+    allow_shared_memory(k_oz_update<32>);
+    allow_shared_memory(k_oz_update<64>);
+    allow_shared_memory(k_lu_coop);
+    done_dev = dev;
 }
 
 }  // namespace
@@ -898,7 +901,7 @@ void launch_cholesky_solve(const Bufs &b, const double *rhs, double *x, cudaStre
     if (n == 0) return;
     const int nblk = div_up(n, NB);
     SFMBA_CUDA(cudaMemsetAsync(b.trsv_ready, 0, sizeof(int) * 2 * (size_t)nblk, s));
-    static int cap_dev = -1, cap = 0;  // co-resident blocks
+    thread_local int cap_dev = -1, cap = 0;  // co-resident blocks
     int dev = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     if (cap_dev != dev) {
@@ -939,7 +942,7 @@ void launch_lu_factor(const Bufs &b, cudaStream_t s) {
     int blocks = 0;
     size_t smem = 0;
     if (!b.lu_by_columns && lu_coop_shape(n, blocks, smem)) {
-        SFMBA_CUDA(cudaFuncSetAttribute(k_lu_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        set_smem_limits();
         launch_coop(k_lu_coop, blocks, blocks, smem, s, b.L, n, b.lu_perm, (const LMState *)b.state,
                     div_up(n, blocks));
         return;

@@ -510,8 +510,8 @@ void run_coop(const Bufs &b, cudaStream_t s, int parity, bool coarse) {
         a.cc = (T *)b.co.cc;
     }
     // Co-resident grid: as many blocks as the widest phase needs, at most
-    // what the GPU holds at once (queried once per instance and device).
-    static int cap_dev = -1, cap = 0;
+    // what the GPU holds at once (queried once per instance, thread and device).
+    thread_local int cap_dev = -1, cap = 0;
     int dev = 0;
     SFMBA_CUDA(cudaGetDevice(&dev));
     if (cap_dev != dev) {
