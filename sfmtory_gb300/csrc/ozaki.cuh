@@ -82,11 +82,9 @@ __device__ __forceinline__ void oz_split_row(const double *__restrict__ row, int
     const unsigned long long b1 = lane + 32 < nb ? (unsigned long long)__double_as_longlong(row[lane + 32]) : 0;
     const int emax = __reduce_max_sync(0xffffffffu, max((int)((b0 & kAbs) >> 52), (int)((b1 & kAbs) >> 52)));
     // max |x| = f 2^e with f in [0.5, 1): |x| 2^-e < 1. A row of zeros and
-    // subnormals, far below any pivot's square root, takes e as if its largest
-    // were normal: the digits are zero.
-    const int e = emax > 0 ? emax - 1022 : 0;
-    const unsigned long long m0 = emax > 0 ? oz_fraction(b0 & kAbs, emax) : 0;
-    const unsigned long long m1 = emax > 0 ? oz_fraction(b1 & kAbs, emax) : 0;
+    // subnormals takes e as if its largest were the smallest normal number.
+    const int scale = max(emax, 1), e = scale - 1022;
+    const unsigned long long m0 = oz_fraction(b0 & kAbs, scale), m1 = oz_fraction(b1 & kAbs, scale);
     const int at = (((lane >> 3) ^ (r & 7)) << 3) + (lane & 7);
     const float s0 = b0 >> 63 ? -1.0f : 1.0f, s1 = b1 >> 63 ? -1.0f : 1.0f;
 #pragma unroll
