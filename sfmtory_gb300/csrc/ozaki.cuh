@@ -14,17 +14,23 @@
 // accumulation holds exactly. The update is
 //   (P P^T)[r, c] = 2^(e_r + e_c) sum_{i,j} 2^-8(i+j) G_ij[r, c],
 //   G_ij = S_i[R] S_j[C]^T,
-// of which the 28 terms with i + j <= 8 are kept (the others lie below
-// 2^-64 of the scale). Products of one weight d = i + j share an FP32
-// accumulator G_d (exact for d <= 5: at most four products, < 2^24; the
-// five of d = 6 may round by a unit, 2^-52 of the scale). The groups
-// d <= 6 are combined exactly in 64-bit integers,
+// of which the 28 terms with i + j <= 8 are kept. Products of one weight d =
+// i + j share an FP32 accumulator G_d (exact for d <= 5: at most four products,
+// < 2^24). The groups d <= 6 are combined exactly in 64-bit integers,
 //   L = 2^32 G_2 + 2^24 G_3 + 2^16 G_4 + 2^8 G_5 + G_6   (< 2^55),
-// the last two in FP32, T = G_7 + G_8 / 2^8 (rounding below 2^-80 of the
-// scale), and
+// the last two in FP32, T = G_7 + G_8 / 2^8, and
 //   (P P^T)[r, c] = 2^(e_r + e_c - 48) (L + T / 2^8)
 // is formed in FP64 (L rounds to 53 bits: the FP64 rounding of the product
 // itself) and subtracted.
+//
+// Error, in units of s = 2^(e_r + e_c) (an entry of P P^T is below 64 s): the
+// weights left out are below 2^-47.3 (six products of weight 9, each < 64 x
+// 255^2 x 2^-72). G_6 may pass 2^24 when digits close to 255 share a sign; its
+// last four accumulations then lose up to two units of 2^-48 each, 2^-45. T
+// rounds below 2^-54, and digits of an entry below 2^-56 of its row's largest
+// are cut off (2^-49 for 64 of both rows). With the result's own rounding the
+// sum stays below 2^-44 (measured: 2^-45.3 for digits of 254 and 255, 2^-46.8 for
+// random ones); 64 multiply-adds in FP64 are within 2^-41.
 //
 // The products run on the fifth-generation tensor cores: one block per 128 x 64
 // tile, its slices fetched by bulk copies in the layout that tcgen05.mma reads
