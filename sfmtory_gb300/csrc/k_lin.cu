@@ -185,16 +185,54 @@ __global__ void __launch_bounds__(kPointInvBlock) k_point_inverse(const T *pt_C,
 }
 
 // rhs_i = -b_i + sum_o Jc~_o^T (Jx~_o h_p): the reduced right-hand side
-// (lib.rs:919-944 and :199-210). W warps per image (a block of 32 W threads
-// per image for W > 1, of four images for W = 1): an image's observations are
-// a chain of gathers, so few images with many observations each want several
-// warps. The FP32 form keeps one (its compensated sums have one order). 47
-// images of 2600 observations, FP64: 47 us with W = 8 against 243.
-template <typename T, int D, int W>
+// (lib.rs:919-944 and :199-210). FP32: one warp per image, whose compensated
+// sums have one order. (With the FP64 form's sums over the lanes below, the
+// compiler leaves the loop fewer registers for its gathers: 400 against 343 us
+// for 40 images of 4800 observations.)
+template <int D>
+__global__ void k_image_rhs32(const float *rec, const int *img_start, const int *img_obs, const int *ob_pt,
+                              const float *pt_h, const unsigned char *pt_ok, const double *img_b, int nI,
+                              double *img_rhs, const unsigned char *img_live) {
+    constexpr int RS = RecLayout<D>::kStride;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (warp >= nI) return;
+    const int i = warp;
+    if (img_live && !img_live[i]) return;
+    float acc[D], comp[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) acc[c] = comp[c] = 0.0f;
+    const int s = img_start[i], e = img_start[i + 1];
+    for (int k = s + lane; k < e; k += 32) {
+        const int o = img_obs[k];
+        const int p = ob_pt[o];
+        if (!pt_ok[p]) continue;
+        const float *r = rec + (size_t)o * RS;
+        const float *h = pt_h + 3 * (size_t)p;
+        const float z0 = r[2] * h[0] + r[3] * h[1] + r[4] * h[2];
+        const float z1 = r[5] * h[0] + r[6] * h[1] + r[7] * h[2];
+#pragma unroll
+        for (int c = 0; c < D; ++c) kahan_add(acc[c], comp[c], r[8 + c] * z0 + r[8 + D + c] * z1);
+    }
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        double v = (double)acc[c] - (double)comp[c];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        if (lane == 0) img_rhs[(size_t)i * D + c] = -img_b[(size_t)i * D + c] + v;
+    }
+}
+
+// FP64: W warps per image (a block of 32 W threads per image for W > 1, of
+// four images for W = 1): an image's observations are a chain of gathers, so
+// few images with many observations each want several warps. 47 images of 2600
+// observations: 47 us with W = 8 against 243.
+template <int D, int W>
 __global__ void __launch_bounds__(W > 1 ? 32 * W : 128)
-    k_image_rhs(const T *rec, const int *img_start, const int *img_obs, const int *ob_pt, const T *pt_h,
-                const unsigned char *pt_ok, const double *img_b, int nI, double *img_rhs,
-                const unsigned char *img_live) {
+    k_image_rhs64(const double *rec, const int *img_start, const int *img_obs, const int *ob_pt, const double *pt_h,
+                  const unsigned char *pt_ok, const double *img_b, int nI, double *img_rhs,
+                  const unsigned char *img_live) {
+    using T = double;
     constexpr int RS = RecLayout<D>::kStride;
     __shared__ double warp_sum[W][16];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -704,11 +742,11 @@ void launch_point_inverse(const Bufs &b, cudaStream_t s) {
 }
 
 namespace {
-template <typename T, int D, int W>
-void image_rhs_w(const Bufs &b, cudaStream_t s) {
-    k_image_rhs<T, D, W><<<W > 1 ? b.nI : div_up(b.nI, 4), W > 1 ? 32 * W : 128, 0, s>>>(
-        (const T *)b.rec, b.img_start, b.img_obs, b.ob_pt, (const T *)b.pt_h, b.pt_ok, b.img_b, b.nI, b.img_rhs,
-        b.img_live);
+template <int D, int W>
+void image_rhs64(const Bufs &b, cudaStream_t s) {
+    k_image_rhs64<D, W><<<W > 1 ? b.nI : div_up(b.nI, 4), W > 1 ? 32 * W : 128, 0, s>>>(
+        (const double *)b.rec, b.img_start, b.img_obs, b.ob_pt, (const double *)b.pt_h, b.pt_ok, b.img_b, b.nI,
+        b.img_rhs, b.img_live);
 }
 }  // namespace
 
@@ -719,10 +757,13 @@ void launch_image_rhs(const Bufs &b, cudaStream_t s) {
         constexpr int D = decltype(dc)::value;
         // Warps by the rounds of 32 observations that a warp is left with (two
         // at least, or the sums over the warps cost more than they save).
-        if (b.mixed) image_rhs_w<float, D, 1>(b, s);
-        else if (per_image >= 512) image_rhs_w<double, D, 8>(b, s);
-        else if (per_image >= 128) image_rhs_w<double, D, 2>(b, s);
-        else image_rhs_w<double, D, 1>(b, s);
+        if (b.mixed)
+            k_image_rhs32<D><<<div_up(b.nI, 4), 128, 0, s>>>((const float *)b.rec, b.img_start, b.img_obs, b.ob_pt,
+                                                             (const float *)b.pt_h, b.pt_ok, b.img_b, b.nI,
+                                                             b.img_rhs, b.img_live);
+        else if (per_image >= 512) image_rhs64<D, 8>(b, s);
+        else if (per_image >= 128) image_rhs64<D, 2>(b, s);
+        else image_rhs64<D, 1>(b, s);
     });
     SFMBA_LAUNCH_CHECK();
 }
