@@ -71,18 +71,27 @@ __global__ void __launch_bounds__(32 * kSchurWarps)
 }
 
 // Chunks of each group, and its partial blocks: its chunks if it has several.
-__global__ void k_schur_count_chunks(const int *group_start, int ngroups, int chunk, int *chunks, int *parts) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g > ngroups) return;
-    const int c = g < ngroups ? (group_start[g + 1] - group_start[g] + chunk - 1) / chunk : 0;
-    chunks[g] = c;
-    parts[g] = c > 1 ? c : 0;
+// Groups are taken by decreasing pair count (t: a group's place in that order),
+// so that the chunks are launched with the shortest last.
+__global__ void k_schur_count_chunks(const int *group_start, const int *group_order, int ngroups, int chunk,
+                                     int *chunks, int *parts) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t > ngroups) return;
+    const int g = t < ngroups ? group_order[t] : 0;
+    const int c = t < ngroups ? (group_start[g + 1] - group_start[g] + chunk - 1) / chunk : 0;
+    chunks[t] = c;
+    parts[t] = c > 1 ? c : 0;
 }
 
-__global__ void k_schur_name_chunks(const int *chunk_off, int ngroups, int *chunk_group) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ngroups) return;
-    for (int c = chunk_off[g]; c < chunk_off[g + 1]; ++c) chunk_group[c] = g;
+// Chunks as {first pair, end, group, partial block or -1 for a whole group}.
+__global__ void k_schur_list_chunks(const int *group_start, const int *group_order, int ngroups, int chunk,
+                                    const int *chunk_off, const int *part_off, int4 *chunks) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ngroups) return;
+    const int g = group_order[t], e = group_start[g + 1], c0 = chunk_off[t], c1 = chunk_off[t + 1];
+    int s = group_start[g];
+    for (int c = c0; c < c1; ++c, s += chunk)
+        chunks[c] = make_int4(s, min(s + chunk, e), g, c1 - c0 == 1 ? -1 : part_off[t] + c - c0);
 }
 
 template <int D>
@@ -106,25 +115,22 @@ __device__ __forceinline__ void store_schur(int i, int j, int r, int c, double v
 template <int D>
 __global__ void __launch_bounds__(64)
     k_schur_chunks(const double *__restrict__ rec, const int2 *__restrict__ pairs,
-                   const int *__restrict__ group_start, const int2 *__restrict__ group_ij, int ngroups, int chunk,
-                   const int *__restrict__ chunk_off, const int *__restrict__ part_off,
-                   const int *__restrict__ chunk_group, const int *__restrict__ ob_pt,
-                   const double *__restrict__ pt_Cinv, const unsigned char *__restrict__ pt_ok,
+                   const int2 *__restrict__ group_ij, const int *__restrict__ nchunks,
+                   const int4 *__restrict__ chunks, const int *__restrict__ ob_pt, const double *__restrict__ pt_Cinv, const unsigned char *__restrict__ pt_ok,
                    const double *__restrict__ img_H, int nID, double *__restrict__ part,
                    double *__restrict__ S_img) {
     using Tile = SchurTile<double, D>;
     __shared__ double sA[2][32][Tile::LDS];
     __shared__ double sP[2][32][Tile::LDS];
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 2 + wl;
-    if (c >= chunk_off[ngroups]) return;
-    const int g = chunk_group[c], k = c - chunk_off[g];
-    const int s = group_start[g] + k * chunk, e = min(s + chunk, group_start[g + 1]);
+    if (c >= *nchunks) return;
+    const int4 ch = chunks[c];
     double out[Tile::RH][Tile::CQ];
-    schur_group<double, D>(rec, pairs, s, e, ob_pt, pt_Cinv, pt_ok, sA[wl], sP[wl], lane, out);
+    schur_group<double, D>(rec, pairs, ch.x, ch.y, ob_pt, pt_Cinv, pt_ok, sA[wl], sP[wl], lane, out);
     if (lane >= Tile::LS) return;
-    const bool whole = chunk_off[g + 1] - chunk_off[g] == 1;
-    double *dst = part + (size_t)(part_off[g] + k) * D * D;
-    const int2 ij = group_ij[g];
+    const bool whole = ch.w < 0;
+    double *dst = part + (size_t)max(ch.w, 0) * D * D;
+    const int2 ij = group_ij[ch.z];
     const int r0 = (lane >> 2) * Tile::RH, c0 = (lane & 3) * Tile::CQ;
 #pragma unroll
     for (int a = 0; a < Tile::RH; ++a)
@@ -137,17 +143,17 @@ __global__ void __launch_bounds__(64)
         }
 }
 
-// Adds the partial blocks of the groups of several chunks, in order; one
-// warp per group.
+// Adds the partial blocks of the groups of several chunks (all among the first
+// ngroups places), in order; one warp per group.
 template <int D>
-__global__ void __launch_bounds__(256) k_schur_combine(const int2 *group_ij, int ngroups, const int *part_off,
-                                                       const double *part, const double *img_H, int nID,
+__global__ void __launch_bounds__(256) k_schur_combine(const int2 *group_ij, const int *group_order, int ngroups,
+                                                       const int *part_off, const double *part, const double *img_H, int nID,
                                                        double *S_img) {
-    const int g = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (g >= ngroups) return;
-    const int a = part_off[g], b = part_off[g + 1];
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (t >= ngroups) return;
+    const int a = part_off[t], b = part_off[t + 1];
     if (a == b) return;
-    const int2 ij = group_ij[g];
+    const int2 ij = group_ij[group_order[t]];
     for (int e = threadIdx.x & 31; e < D * D; e += 32) {
         double v = 0.0;
         for (int k = a; k < b; ++k) v += part[(size_t)k * D * D + e];
@@ -685,12 +691,15 @@ void launch_schur_pairs(const Bufs &b, cudaStream_t s) {
                 (const float *)b.pt_Cinv, b.pt_ok, b.img_H, b.nID, b.S_img);
         else {
             k_schur_chunks<D><<<div_up(b.schur_max_chunks, 2), 64, 0, s>>>(
-                (const double *)b.rec, b.pairs, b.group_start, b.group_ij, b.ngroups, b.schur_chunk,
-                b.schur_chunk_off, b.schur_part_off, b.schur_chunk_group, b.ob_pt, (const double *)b.pt_Cinv,
-                b.pt_ok, b.img_H, b.nID, b.schur_part, b.S_img);
+                (const double *)b.rec, b.pairs, b.group_ij, b.schur_chunk_off + b.ngroups, b.schur_chunks, b.ob_pt,
+                (const double *)b.pt_Cinv, b.pt_ok, b.img_H, b.nID, b.schur_part, b.S_img);
             SFMBA_LAUNCH_CHECK();
-            k_schur_combine<D><<<div_up(b.ngroups, 8), 256, 0, s>>>(b.group_ij, b.ngroups, b.schur_part_off,
-                                                                    b.schur_part, b.img_H, b.nID, b.S_img);
+            // Groups of several chunks come first and have more pairs than a chunk each.
+            const int several = (int)std::min<long long>(b.ngroups, b.npairs / (b.schur_chunk + 1));
+            if (several > 0)
+                k_schur_combine<D><<<div_up(several, 8), 256, 0, s>>>(b.group_ij, b.group_order, several,
+                                                                      b.schur_part_off, b.schur_part, b.img_H, b.nID,
+                                                                      b.S_img);
         }
     });
     SFMBA_LAUNCH_CHECK();
@@ -704,11 +713,17 @@ int schur_chunk_pairs(long long npairs, int sms) {
     return (int)std::min<long long>(256, std::max<long long>(32, c));
 }
 
-// Chunk offsets and names of the current groups (temp: CUB scratch).
-void launch_schur_chunks(const Bufs &b, void *temp, size_t temp_bytes, cudaStream_t s) {
+// Chunks of the current groups (temp: CUB scratch). Where the groups alone are
+// as many warps as the chunks aim at, none of two rounds of pairs is cut (60
+// images of 30 points each that most of them see: 105 us cut at 32 pairs, 96 at
+// 64 and more).
+void launch_schur_chunks(Bufs &b, int sms, void *temp, size_t temp_bytes, cudaStream_t s) {
     if (b.ngroups == 0) return;
-    k_schur_count_chunks<<<div_up(b.ngroups + 1, 256), 256, 0, s>>>(b.group_start, b.ngroups, b.schur_chunk,
-                                                                    b.schur_chunk_off, b.schur_part_off);
+    if (b.ngroups >= 8 * sms)
+        b.schur_chunk = std::max(b.schur_chunk, 64);
+    b.schur_max_chunks = (int)(b.npairs / b.schur_chunk + b.ngroups);
+    k_schur_count_chunks<<<div_up(b.ngroups + 1, 256), 256, 0, s>>>(
+        b.group_start, b.group_order, b.ngroups, b.schur_chunk, b.schur_chunk_off, b.schur_part_off);
     SFMBA_LAUNCH_CHECK();
     for (int *v : {b.schur_chunk_off, b.schur_part_off}) {
         size_t need = 0;
@@ -716,7 +731,8 @@ void launch_schur_chunks(const Bufs &b, void *temp, size_t temp_bytes, cudaStrea
         if (need > temp_bytes) throw Error(SFMBA_ERR_INTERNAL, "chunk scan temp too small");
         SFMBA_CUDA(cub::DeviceScan::ExclusiveSum(temp, need, v, v, b.ngroups + 1, s));
     }
-    k_schur_name_chunks<<<div_up(b.ngroups, 256), 256, 0, s>>>(b.schur_chunk_off, b.ngroups, b.schur_chunk_group);
+    k_schur_list_chunks<<<div_up(b.ngroups, 256), 256, 0, s>>>(b.group_start, b.group_order, b.ngroups, b.schur_chunk,
+                                                               b.schur_chunk_off, b.schur_part_off, b.schur_chunks);
     SFMBA_LAUNCH_CHECK();
 }
 

@@ -131,9 +131,9 @@ struct Bufs {
     // (launch_schur_chunks); partial blocks of the groups of several chunks.
     int schur_chunk = 0;                 // 0: one warp per group
     int schur_max_chunks = 0;
-    int *schur_chunk_off = nullptr;      // [ngroups + 1] first chunk of each group
-    int *schur_part_off = nullptr;       // [ngroups + 1] first partial block of each group
-    int *schur_chunk_group = nullptr;    // [schur_max_chunks]
+    int *schur_chunk_off = nullptr;      // [ngroups + 1] first chunk of each group, in group_order
+    int *schur_part_off = nullptr;       // [ngroups + 1] first partial block of each group, in group_order
+    int4 *schur_chunks = nullptr;        // [schur_max_chunks] k_schur_list_chunks
     double *schur_part = nullptr;        // [partial blocks][D * D]
     long long npairs = 0;
     int ngroups = 0;
@@ -328,7 +328,7 @@ void launch_jacobian_probe(const JacProbe &q, bool fp32, cudaStream_t s);
 // ---- dense reduced system (k_dense.cu)
 void launch_schur_pairs(const Bufs &b, cudaStream_t s);
 int schur_chunk_pairs(long long npairs, int sms);
-void launch_schur_chunks(const Bufs &b, void *temp, size_t temp_bytes, cudaStream_t s);
+void launch_schur_chunks(Bufs &b, int sms, void *temp, size_t temp_bytes, cudaStream_t s);
 // Slots that more images map to than this are folded through the list of image pairs (k_dense.cu).
 constexpr int kFoldList = 32;
 size_t shared_fold_temp_bytes(long long nkeys);

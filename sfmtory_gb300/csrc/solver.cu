@@ -1346,9 +1346,9 @@ class Solver {
             // one image pair per group and one chunk more than whole ones per group.
             const bool fp64_schur = !batch && (!mixed || polish);
             const long long max_groups = std::min<long long>(b.npairs, (long long)nI * (nI + 1) / 2);
+            int sms = 0;
+            SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx_.device));
             if (fp64_schur) {
-                int sms = 0;
-                SFMBA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx_.device));
                 b.schur_chunk = schur_chunk_pairs(b.npairs, sms);
                 b.schur_max_chunks = (int)(b.npairs / b.schur_chunk + max_groups);
             }
@@ -1366,12 +1366,12 @@ class Solver {
                 if (fp64_schur) {
                     b.schur_chunk_off = P.take<int>(max_groups + 1);
                     b.schur_part_off = P.take<int>(max_groups + 1);
-                    b.schur_chunk_group = P.take<int>(b.schur_max_chunks);
+                    b.schur_chunks = P.take<int4>(b.schur_max_chunks);
                     b.schur_part = P.take<double>((size_t)(2 * b.npairs / b.schur_chunk + 1) * D * D);
                 }
             }
             build_pairs(b, pair_scan, ka, kb, vb, pt, ptemp, d_ng, s_);
-            if (fp64_schur) launch_schur_chunks(b, pt, ptemp, s_);
+            if (fp64_schur) launch_schur_chunks(b, sms, pt, ptemp, s_);
             if (!batch) setup_shared_fold();
             const size_t simg = batch ? (size_t)batch->simg_total : (size_t)nID * nID;
             SFMBA_CUDA(cudaMemsetAsync(b.S_img, 0, sizeof(double) * simg, s_));
