@@ -32,25 +32,25 @@ namespace {
 constexpr int kSchurWarps = 4;
 
 // The FP32 reduction, one warp per image pair.
-template <typename T, int D>
+template <int D>
 __global__ void __launch_bounds__(32 * kSchurWarps)
-    k_schur_pairs(const T *__restrict__ rec, const int2 *__restrict__ pairs,
+    k_schur_pairs(const float *__restrict__ rec, const int2 *__restrict__ pairs,
                   const int *__restrict__ group_start, const int2 *__restrict__ group_ij,
                   const int *__restrict__ group_order, int ngroups,
-                  const int *__restrict__ ob_pt, const T *__restrict__ pt_Cinv,
+                  const int *__restrict__ ob_pt, const float *__restrict__ pt_Cinv,
                   const unsigned char *__restrict__ pt_ok, const double *__restrict__ img_H, int nID,
                   double *__restrict__ S_img) {
     constexpr int W = kSchurWarps;
-    using Tile = SchurTile<T, D>;
-    __shared__ T sA[W][32][Tile::LDS];
-    __shared__ T sP[W][32][Tile::LDS];
+    using Tile = SchurTile<float, D>;
+    __shared__ float sA[W][32][Tile::LDS];
+    __shared__ float sP[W][32][Tile::LDS];
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (blockIdx.x * W + wl >= ngroups) return;
     const int g = group_order[blockIdx.x * W + wl];
     const int2 ij = group_ij[g];
     double out[Tile::RH][Tile::CQ];
-    schur_group<T, D>(rec, pairs, group_start[g], group_start[g + 1], ob_pt, pt_Cinv, pt_ok, sA[wl], sP[wl], lane,
-                      out);
+    schur_group<float, D>(rec, pairs, group_start[g], group_start[g + 1], ob_pt, pt_Cinv, pt_ok, sA[wl], sP[wl],
+                          lane, out);
     if (lane >= Tile::LS) return;
     const int i = ij.x, j = ij.y;
     const int r0 = (lane >> 2) * Tile::RH, c0 = (lane & 3) * Tile::CQ;
@@ -686,7 +686,7 @@ void launch_schur_pairs(const Bufs &b, cudaStream_t s) {
     dispatch_D(b.D, [&](auto dc) {
         constexpr int D = decltype(dc)::value;
         if (b.mixed)
-            k_schur_pairs<float, D><<<div_up(b.ngroups, kSchurWarps), 32 * kSchurWarps, 0, s>>>(
+            k_schur_pairs<D><<<div_up(b.ngroups, kSchurWarps), 32 * kSchurWarps, 0, s>>>(
                 (const float *)b.rec, b.pairs, b.group_start, b.group_ij, b.group_order, b.ngroups, b.ob_pt,
                 (const float *)b.pt_Cinv, b.pt_ok, b.img_H, b.nID, b.S_img);
         else {
@@ -815,13 +815,6 @@ LookAhead &look_ahead() {
 
 }  // namespace
 
-// Blocked right-looking Cholesky with a look-ahead of one panel: after the
-// panel of block k, the tile column of block k + 1 is updated first; then
-// the diagonal factor, panel (and slices) of block k + 1 run on a second
-// stream while the rest of block k's trailing update runs on s. The
-// diagonal factor is the serial part (one block, FP64-pipe bound), so it
-// hides behind the bulk update. Tensor-core updates read the panel slices of
-// their own step: two slice buffers alternate by step.
 // Cooperative launch of kernel k with `want` blocks of 256 threads at most
 // what the GPU holds at once (cap: co-resident blocks, queried once per
 // device by the caller); false when none can be resident.
@@ -853,6 +846,13 @@ int coop_capacity(K k, size_t smem) {
     return per_sm * sms;
 }
 
+// Blocked right-looking Cholesky with a look-ahead of one panel: after the
+// panel of block k, the tile column of block k + 1 is updated first; then
+// the diagonal factor, panel (and slices) of block k + 1 run on a second
+// stream while the rest of block k's trailing update runs on s. The
+// diagonal factor is the serial part (one cluster of three blocks, FP64-pipe
+// bound), so it hides behind the bulk update. Tensor-core updates read the panel slices of
+// their own step: two slice buffers alternate by step.
 void launch_cholesky(const Bufs &b, cudaStream_t s) {
     set_smem_limits();
     const int n = b.n;
