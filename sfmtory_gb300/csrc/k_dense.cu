@@ -108,10 +108,10 @@ __device__ __forceinline__ void store_schur(int i, int j, int r, int c, double v
 // The FP64 reduction, one warp per chunk of a group's pairs: a warp's FP64
 // instruction takes its sub-partition for 65 cycles, so one warp per group
 // left a few long groups (an image with itself: all its observations) to run
-// alone. 47 OPENCV images, 120 000 observations: 0.67 against 1.71
-// ms; 16 images that see all of 2000 points: 0.21 against 0.80 ms. The FP32
-// form keeps one warp per group: its compensated sum over a group's rounds
-// has one order.
+// alone. 47 OPENCV images, 120 000 observations: 0.59 against 1.71
+// ms; 16 images that see all of 2000 points: 0.21 against 0.80 ms; 500 images
+// of 240 observations, 4500 groups: 0.73 either way. The FP32 form keeps one
+// warp per group: its compensated sum over a group's rounds has one order.
 template <int D>
 __global__ void __launch_bounds__(64)
     k_schur_chunks(const double *__restrict__ rec, const int2 *__restrict__ pairs,
